@@ -316,7 +316,7 @@ int b200shm_span_amo(int amo, int dtype, int G, const uint64_t *bases, int pe_st
 
 /* One reduction of a batch: the arguments of b200shm_reduce.  `lanes` and
  * `tile` are outputs of b200shm_batch_create: the lanes per 16-byte column
- * and the units per tile the autotuner chose (0 = this reduction runs as
+ * and the units per tile, at most, the autotuner chose (0 = this reduction runs as
  * its own launch because the batch kernels do not cover its
  * (dtype, op, algo, size)); `algo` is rewritten when it was AUTO. */
 typedef struct b200shm_reduce_desc {
@@ -350,12 +350,13 @@ typedef struct b200shm_batch b200shm_batch;
  * plan. */
 int b200shm_batch_create(b200shm_reduce_desc *descs, uint64_t n, int flags,
                          b200shm_batch **out);
-/* Run the whole batch: one persistent launch per (type, op, combine order)
- * group, the groups overlapping on side streams, plus one launch that
- * replays order-dependent float MIN/MAX elements and one launch per
- * reduction the batch kernels do not cover.  With B200SHM_BATCH_GRAPH the
- * run is a single CUDA graph launch.  Runs of one batch must not overlap
- * on the GPU (they share its tile counters). */
+/* Run the whole batch: the tiles of all its reductions in two launches side
+ * by side (float trees; everything else), plus one launch that replays
+ * order-dependent float MIN/MAX elements and one launch per reduction the
+ * batch kernels do not cover.  With B200SHM_BATCH_GRAPH the run is a single
+ * CUDA graph launch.  Runs of batches with float MIN/MAX must not overlap
+ * on the GPU (they share the engine's list of deferred elements), nor runs
+ * of one batch. */
 int b200shm_batch_run(b200shm_batch *batch, void *stream);
 int b200shm_batch_destroy(b200shm_batch *batch);
 /* create + run + destroy. */

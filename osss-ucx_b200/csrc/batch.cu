@@ -5,12 +5,12 @@
  * The reference can only issue shcoll_<T>_<op>_reduce_<algo> calls one
  * after the other (src/shcoll/src/reduce.c:1078-1102), each a full
  * algorithm with its own synchronisation.  Here a batch is planned once:
- * every descriptor is cut into tiles of 16-byte columns, descriptors are
- * sorted into groups of one (type slot, op, combine order), and each group
- * runs as ONE persistent kernel specialised for it that takes tiles from a
- * counter.  Groups are spread over a few side streams so that one group's
- * tail overlaps the next group's start; with B200SHM_BATCH_GRAPH the whole
- * run is captured once into a CUDA graph.
+ * every descriptor is cut into tiles of 16-byte columns, and the tiles of
+ * the whole batch, whatever their type, op and combine order, run as two
+ * launches side by side, one CTA per tile: the order-free reductions (and
+ * left folds) in one, the float trees, which need more registers and a
+ * shared-memory stack, in the other.  With B200SHM_BATCH_GRAPH the run is
+ * captured once into a CUDA graph.
  *
  * Every result is bit-identical to b200shm_reduce on the same descriptor:
  * a lane combines its members in the same order as the per-call kernels
@@ -34,11 +34,10 @@
 #include <vector>
 
 #include "internal.cuh"
-/* The batch kernels keep write-back stores and L1-bypassing loads: with
- * the streaming (evict-first) policy of the per-call kernels the batching
- * workload ran 2.63-2.66 ms against 2.615-2.620. */
+/* L1-bypassing loads, streaming stores: 2048 reductions over 256 teams
+ * (2.08 GB) ran in 413.6 us with streaming stores, 417.4 with write-back. */
 #define B200_LD_OP "ld.global.nc.L1::no_allocate"
-#define B200_ST_OP "st.global"
+#define B200_ST_OP "st.global.cs"
 #include "reduce_core.cuh"
 
 namespace b200 {
@@ -68,15 +67,48 @@ struct BDesc {
   int id;              /* index of the caller's descriptor */
 };
 
+/* One tile, as its CTA reads it: a range of columns of one descriptor. */
+struct alignas(16) BTile {
+  const char *src;   /* member 0's source at the tile's first element       */
+  char *dst;         /* member 0's dest there                               */
+  uint64_t step;     /* bytes between consecutive members                   */
+  uint64_t e0;       /* the tile's first element, counted in the descriptor */
+  uint32_t di;       /* the descriptor (its index in the sorted plan)       */
+  uint32_t cnt;      /* 16-byte packs (vec), else elements                  */
+  uint16_t P, kid;
+  uint8_t G, vec;    /* lanes per column                                    */
+  uint8_t tail, pad; /* elements after the last pack, served by this tile   */
+};
+static_assert(sizeof(BTile) == 48, "a tile is three 16-byte loads");
+
 struct BPlan {
   const BDesc *d;
-  const uint32_t *prefix; /* ndesc + 1 tile prefix sums */
-  const uint2 *tile_map;  /* per tile of the plan: (descriptor, tile within it) */
-  uint32_t ndesc, total;
+  const BTile *tiles;
   unsigned long long *fix_list, *fix_count;
   unsigned long long fix_cap;
   int *status;
 };
+
+/* The member step, as a value the compiler cannot multiply ahead: eight
+ * precomputed multiples of it cost a lane 16 registers, eight additions
+ * cost next to nothing beside eight loads. */
+__device__ __forceinline__ uint64_t opaque(uint64_t v) {
+  asm volatile("" : "+l"(v));
+  return v;
+}
+
+/* A column's operand classes (fclass, 3 bits an element) in one register. */
+template <class PK>
+__device__ __forceinline__ unsigned pack_class(const PK &v) {
+  unsigned c = 0;
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(v.x) / sizeof(v.x[0])); i++) c |= fclass(v.x[i]) << (3 * i);
+  return c;
+}
+/* some element saw a NaN, or zeros of both signs */
+__device__ __forceinline__ bool pack_ambiguous(unsigned c) {
+  return ((c & 01111u) | ((c >> 1) & (c >> 2) & 01111u)) != 0;
+}
 
 /* A lane's stack of complete subtrees lives in shared memory, one 32-bit
  * word per thread per row ([level][word][thread]), so that a warp's
@@ -100,59 +132,59 @@ __device__ __forceinline__ PK stk_get(const uint32_t *stk, int L) {
   return v;
 }
 
-/* One tile: units [u0, u0+cnt) of descriptor d, a unit being a V-element
- * pack.  G lanes share a column; lane g reduces leaves [l0, l1) (members
- * [m0, m1), a butterfly leaf's extra member included), the G partials are
- * combined with shuffles over masks 1, 2, ..., G/2 (the tree's top
- * levels), and each lane stores the result to its own members. */
+/* cnt units of V elements from element `at` of the tile (its units, or the
+ * elements after them).  G lanes share a column; lane g reduces leaves
+ * [l0, l1) (members [m0, m1), a butterfly leaf's extra member included),
+ * the G partials are combined with shuffles over masks 1, 2, ..., G/2 (the
+ * tree's top levels), and each lane stores the result to its own members. */
 template <class T, int OP, int ORDER, bool MM, int V>
-__device__ void run_tile(const BDesc &d, uint32_t di, uint64_t u0, uint64_t cnt, const BPlan &p,
-                         uint32_t *stk) {
+__device__ __forceinline__ void run_tile(const BTile &d, uint64_t at, uint32_t cnt, const BPlan &p,
+                                         uint32_t *stk) {
   typedef Pack<T, V> PK;
   const int G = d.G;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kBatchThreads >> 5;
-  const int g = lane & (G - 1), cw = lane / G, cpw = 32 / G;
+  const int lane = threadIdx.x & 31, nw = kBatchThreads >> 5;
+  /* a tile's trailing elements go to the last warps, which a short tile idles */
+  const int warp = V == 1 ? nw - 1 - (threadIdx.x >> 5) : threadIdx.x >> 5;
+  const int lgG = __ffs(G) - 1;
+  const int g = lane & (G - 1), cw = lane >> lgG, cpw = 32 >> lgG;
   const int P = d.P;
-  const int nleaves = ORDER == ORD_BUTTERFLY ? d.p2s : P;
-  const int l0 = (int)((long long)g * nleaves / G), l1 = (int)((long long)(g + 1) * nleaves / G);
+  const int lg = 31 - __clz(P), p2s = 1 << lg;
+  const int nleaves = ORDER == ORD_BUTTERFLY ? p2s : P;
+  const int l0 = (g * nleaves) >> lgG, l1 = ((g + 1) * nleaves) >> lgG;
   /* the member holding leaf q: ceil(q * P / p2s) for the butterfly */
   auto member_of = [&](int q) -> int {
-    return ORDER == ORD_BUTTERFLY ? (int)(((long long)q * P + d.p2s - 1) >> d.logp2s) : q;
+    return ORDER == ORD_BUTTERFLY ? (q * P + p2s - 1) >> lg : q;
   };
   const int m0 = member_of(l0), m1 = member_of(l1);
   auto comb = [](const PK &lo, const PK &hi) {
     if constexpr (ORDER == ORD_BINOMIAL) return papply<OP>(hi, lo);
     else return papply<OP>(lo, hi);
   };
-  for (uint64_t base = (uint64_t)warp * cpw; base < cnt; base += (uint64_t)nw * cpw) {
-    const uint64_t col = base + cw;
+  for (uint32_t base = warp * cpw; base < cnt; base += nw * cpw) {
+    const uint32_t col = base + cw;
     const bool live = col < cnt;
-    const uint64_t e0 = (u0 + (live ? col : 0)) * V;
+    const uint64_t e0 = at + (uint64_t)(live ? col : 0) * V;
     const char *src = d.src + e0 * sizeof(T);
     PK r;
-    unsigned cls[V];
-#pragma unroll
-    for (int i = 0; i < V; i++) cls[i] = 0;
+    unsigned cls = 0;
     if (live) {
       if constexpr (ORDER == ORD_CHAIN) {
-        r = ld_pack<T, V>(src + (uint64_t)m0 * d.step);
-        if constexpr (MM) {
-#pragma unroll
-          for (int i = 0; i < V; i++) cls[i] = fclass(r.x[i]);
-        }
+        const char *q = src + (uint64_t)m0 * d.step;
+        r = ld_pack<T, V>(q);
+        if constexpr (MM) cls = pack_class(r);
         for (int j = m0 + 1; j < m1; j += 8) {
           PK x[8];
+          const uint64_t step = opaque(d.step);
 #pragma unroll
-          for (int u = 0; u < 8; u++)
-            if (j + u < m1) x[u] = ld_pack<T, V>(src + (uint64_t)(j + u) * d.step);
+          for (int u = 0; u < 8; u++) {
+            q += step;
+            if (j + u < m1) x[u] = ld_pack<T, V>(q);
+          }
 #pragma unroll
           for (int u = 0; u < 8; u++)
             if (j + u < m1) {
               r = papply<OP>(r, x[u]);
-              if constexpr (MM) {
-#pragma unroll
-                for (int i = 0; i < V; i++) cls[i] |= fclass(x[u].x[i]);
-              }
+              if constexpr (MM) cls |= pack_class(x[u]);
             }
         }
       } else {
@@ -177,19 +209,24 @@ __device__ void run_tile(const BDesc &d, uint32_t di, uint64_t u0, uint64_t cnt,
           constexpr int KB = decltype(kb_c)::value;
           constexpr bool EX = decltype(ex_c)::value;
           constexpr int LB = KB == 8 ? 3 : 2;
+          const char *q = src + (uint64_t)m0 * d.step; /* leaves in member order */
           for (int qb = l0; qb < l1; qb += KB) {
             const int k = l1 - qb < KB ? l1 - qb : KB;
+            const uint64_t step = opaque(d.step);
             PK x[KB], e[EX ? KB : 1];
             bool ex[KB];
 #pragma unroll
             for (int u = 0; u < KB; u++) {
               ex[u] = false;
               if (u < k) {
-                const int mo = member_of(qb + u);
-                x[u] = ld_pack<T, V>(src + (uint64_t)mo * d.step);
+                x[u] = ld_pack<T, V>(q);
+                q += step;
                 if constexpr (EX) {
-                  ex[u] = member_of(qb + u + 1) - mo == 2;
-                  if (ex[u]) e[u] = ld_pack<T, V>(src + (uint64_t)(mo + 1) * d.step);
+                  ex[u] = member_of(qb + u + 1) - member_of(qb + u) == 2;
+                  if (ex[u]) {
+                    e[u] = ld_pack<T, V>(q);
+                    q += step;
+                  }
                 }
               }
             }
@@ -212,7 +249,7 @@ __device__ void run_tile(const BDesc &d, uint32_t di, uint64_t u0, uint64_t cnt,
             }
           }
         };
-        if (ORDER == ORD_BUTTERFLY && P != d.p2s)
+        if (ORDER == ORD_BUTTERFLY && P != p2s)
           leaves(std::integral_constant<int, 4>{}, std::true_type{});
         else
           leaves(std::integral_constant<int, 8>{}, std::false_type{});
@@ -233,22 +270,16 @@ __device__ void run_tile(const BDesc &d, uint32_t di, uint64_t u0, uint64_t cnt,
     for (int m = 1; m < G; m <<= 1) {
       const PK o = shfl_xor_pack<T, V>(r, m);
       r = (g & m) ? comb(o, r) : comb(r, o);
-      if constexpr (MM) {
-#pragma unroll
-        for (int i = 0; i < V; i++) cls[i] |= __shfl_xor_sync(0xffffffffu, cls[i], m);
-      }
+      if constexpr (MM) cls |= __shfl_xor_sync(0xffffffffu, cls, m);
     }
     if (!live) continue;
     if constexpr (MM) {
-      bool amb = false;
-#pragma unroll
-      for (int i = 0; i < V; i++) amb |= ambiguous(cls[i]);
-      if (amb) { /* deferred: (descriptor, element) pairs, dests untouched */
+      if (pack_ambiguous(cls)) { /* deferred: (descriptor, element) pairs, dests untouched */
         if (g == 0) {
           const unsigned long long slot = atomicAdd(p.fix_count, (unsigned long long)V);
           for (int i = 0; i < V; i++) {
             if (slot + i < p.fix_cap)
-              p.fix_list[slot + i] = ((unsigned long long)di << 40) | (e0 + i);
+              p.fix_list[slot + i] = ((unsigned long long)d.di << 40) | (d.e0 + e0 + i);
             else
               atomicOr(p.status, (int)B200SHM_STATUS_FIX_OVERFLOW);
           }
@@ -256,8 +287,8 @@ __device__ void run_tile(const BDesc &d, uint32_t di, uint64_t u0, uint64_t cnt,
         continue;
       }
     }
-    char *dst = d.dst + e0 * sizeof(T);
-    for (int j = m0; j < m1; j++) st_pack<T, V>(dst + (uint64_t)j * d.step, r);
+    char *dst = d.dst + e0 * sizeof(T) + (uint64_t)m0 * d.step;
+    for (int j = m0; j < m1; j++, dst += d.step) st_pack<T, V>(dst, r);
   }
 }
 
@@ -266,84 +297,94 @@ __device__ void run_tile(const BDesc &d, uint32_t di, uint64_t u0, uint64_t cnt,
  * batches of 8/U per column), and butterflies whose lanes hold at most 2
  * leaves (combined in registers per column, extras loaded alongside). */
 template <class T, int OP, int ORDER, bool MM, int V, int U>
-__device__ void run_tile_multi(const BDesc &d, uint32_t di, uint64_t u0, uint64_t cnt,
-                               const BPlan &p) {
+__device__ __forceinline__ void run_tile_multi(const BTile &d, uint64_t at, uint32_t cnt,
+                                               const BPlan &p) {
   typedef Pack<T, V> PK;
   const int G = d.G;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = kBatchThreads >> 5;
-  const int g = lane & (G - 1), cw = lane / G, cpw = 32 / G;
+  constexpr uint32_t UB = (uint32_t)(V * sizeof(T));
+  const int lane = threadIdx.x & 31, nw = kBatchThreads >> 5;
+  const int warp = V == 1 ? nw - 1 - (threadIdx.x >> 5) : threadIdx.x >> 5;
+  const int lgG = __ffs(G) - 1;
+  const int g = lane & (G - 1), cw = lane >> lgG, cpw = 32 >> lgG;
   const int P = d.P;
-  const int nleaves = ORDER == ORD_BUTTERFLY ? d.p2s : P;
-  const int l0 = (int)((long long)g * nleaves / G), l1 = (int)((long long)(g + 1) * nleaves / G);
+  const int lg = 31 - __clz(P), p2s = 1 << lg;
+  const int nleaves = ORDER == ORD_BUTTERFLY ? p2s : P;
+  const int l0 = (g * nleaves) >> lgG, l1 = ((g + 1) * nleaves) >> lgG;
   auto member_of = [&](int q) -> int {
-    return ORDER == ORD_BUTTERFLY ? (int)(((long long)q * P + d.p2s - 1) >> d.logp2s) : q;
+    return ORDER == ORD_BUTTERFLY ? (q * P + p2s - 1) >> lg : q;
   };
+  const char *tsrc = d.src + at * sizeof(T);
+  char *tdst = d.dst + at * sizeof(T);
   const int m0 = member_of(l0), m1 = member_of(l1);
   auto comb = [](const PK &lo, const PK &hi) { return papply<OP>(lo, hi); };
-  for (uint64_t base = (uint64_t)warp * cpw * U; base < cnt; base += (uint64_t)nw * cpw * U) {
+  for (uint32_t base = warp * cpw * U; base < cnt; base += nw * cpw * U) {
     PK r[U];
-    unsigned cls[U][V];
+    unsigned cls[U];
     bool live[U];
-    const char *src[U];
+    /* column k of this lane is `gap` bytes past column k - 1 */
+    const char *src0 = tsrc + (uint64_t)(base + cw) * UB;
+    const uint64_t gap = (uint64_t)cpw * UB;
 #pragma unroll
     for (int k = 0; k < U; k++) {
-      const uint64_t col = base + cw + (uint64_t)k * cpw;
-      live[k] = col < cnt;
-      src[k] = d.src + (u0 + (live[k] ? col : 0)) * V * sizeof(T);
-#pragma unroll
-      for (int i = 0; i < V; i++) cls[k][i] = 0;
+      live[k] = base + cw + k * cpw < cnt;
+      cls[k] = 0;
     }
     if constexpr (ORDER == ORD_CHAIN) {
-      constexpr int MB = 8 / U; /* members per batch, per column */
+      /* members per batch, per column, beyond the first: a lane of four
+       * columns has two members at most, one of two columns four */
+      constexpr int MB = U == 4 ? 1 : 3;
+      const char *q = src0 + (uint64_t)m0 * d.step;
 #pragma unroll
       for (int k = 0; k < U; k++)
         if (live[k]) {
-          r[k] = ld_pack<T, V>(src[k] + (uint64_t)m0 * d.step);
-          if constexpr (MM) {
-#pragma unroll
-            for (int i = 0; i < V; i++) cls[k][i] = fclass(r[k].x[i]);
-          }
+          r[k] = ld_pack<T, V>(q + k * gap);
+          if constexpr (MM) cls[k] = pack_class(r[k]);
         }
       for (int j = m0 + 1; j < m1; j += MB) {
         PK x[U][MB];
+        const uint64_t step = opaque(d.step);
 #pragma unroll
-        for (int k = 0; k < U; k++)
+        for (int u = 0; u < MB; u++) {
+          q += step;
 #pragma unroll
-          for (int u = 0; u < MB; u++)
-            if (live[k] && j + u < m1) x[k][u] = ld_pack<T, V>(src[k] + (uint64_t)(j + u) * d.step);
+          for (int k = 0; k < U; k++)
+            if (live[k] && j + u < m1) x[k][u] = ld_pack<T, V>(q + k * gap);
+        }
 #pragma unroll
         for (int k = 0; k < U; k++)
 #pragma unroll
           for (int u = 0; u < MB; u++)
             if (live[k] && j + u < m1) {
               r[k] = papply<OP>(r[k], x[k][u]);
-              if constexpr (MM) {
-#pragma unroll
-                for (int i = 0; i < V; i++) cls[k][i] |= fclass(x[k][u].x[i]);
-              }
+              if constexpr (MM) cls[k] |= pack_class(x[k][u]);
             }
       }
     } else { /* butterfly, l1 - l0 in {1, 2} leaves per lane */
       const int n = l1 - l0;
       PK x[U][2], e[U][2];
-      bool ex[U][2];
+      bool ex[2];
+      const char *q = src0 + (uint64_t)m0 * d.step;
 #pragma unroll
-      for (int k = 0; k < U; k++)
+      for (int u = 0; u < 2; u++) {
+        ex[u] = u < n && member_of(l0 + u + 1) - member_of(l0 + u) == 2;
+        if (u < n) {
 #pragma unroll
-        for (int u = 0; u < 2; u++) {
-          ex[k][u] = false;
-          if (live[k] && u < n) {
-            const int own = member_of(l0 + u);
-            x[k][u] = ld_pack<T, V>(src[k] + (uint64_t)own * d.step);
-            ex[k][u] = member_of(l0 + u + 1) - own == 2;
-            if (ex[k][u]) e[k][u] = ld_pack<T, V>(src[k] + (uint64_t)(own + 1) * d.step);
-          }
+          for (int k = 0; k < U; k++)
+            if (live[k]) x[k][u] = ld_pack<T, V>(q + k * gap);
+          q += d.step;
         }
+        if (ex[u]) {
+#pragma unroll
+          for (int k = 0; k < U; k++)
+            if (live[k]) e[k][u] = ld_pack<T, V>(q + k * gap);
+          q += d.step;
+        }
+      }
 #pragma unroll
       for (int k = 0; k < U; k++) {
 #pragma unroll
         for (int u = 0; u < 2; u++)
-          if (ex[k][u]) x[k][u] = papply<OP>(e[k][u], x[k][u]); /* op(extra, own) */
+          if (ex[u]) x[k][u] = papply<OP>(e[k][u], x[k][u]); /* op(extra, own) */
         r[k] = n == 1 ? x[k][0] : comb(x[k][0], x[k][1]);
       }
     }
@@ -352,26 +393,20 @@ __device__ void run_tile_multi(const BDesc &d, uint32_t di, uint64_t u0, uint64_
       for (int k = 0; k < U; k++) {
         const PK o = shfl_xor_pack<T, V>(r[k], m);
         r[k] = (g & m) ? comb(o, r[k]) : comb(r[k], o);
-        if constexpr (MM) {
-#pragma unroll
-          for (int i = 0; i < V; i++) cls[k][i] |= __shfl_xor_sync(0xffffffffu, cls[k][i], m);
-        }
+        if constexpr (MM) cls[k] |= __shfl_xor_sync(0xffffffffu, cls[k], m);
       }
     }
 #pragma unroll
     for (int k = 0; k < U; k++) {
       if (!live[k]) continue;
-      const uint64_t e0 = (uint64_t)(src[k] - d.src) / sizeof(T);
       if constexpr (MM) {
-        bool amb = false;
-#pragma unroll
-        for (int i = 0; i < V; i++) amb |= ambiguous(cls[k][i]);
-        if (amb) { /* deferred: (descriptor, element) pairs, dests untouched */
+        if (pack_ambiguous(cls[k])) { /* deferred: (descriptor, element) pairs, dests untouched */
           if (g == 0) {
             const unsigned long long slot = atomicAdd(p.fix_count, (unsigned long long)V);
+            const uint64_t e0 = at + (uint64_t)(base + cw + k * cpw) * V;
             for (int i = 0; i < V; i++) {
               if (slot + i < p.fix_cap)
-                p.fix_list[slot + i] = ((unsigned long long)di << 40) | (e0 + i);
+                p.fix_list[slot + i] = ((unsigned long long)d.di << 40) | (d.e0 + e0 + i);
               else
                 atomicOr(p.status, (int)B200SHM_STATUS_FIX_OVERFLOW);
             }
@@ -379,55 +414,100 @@ __device__ void run_tile_multi(const BDesc &d, uint32_t di, uint64_t u0, uint64_
           continue;
         }
       }
-      char *dst = d.dst + e0 * sizeof(T);
-      for (int j = m0; j < m1; j++) st_pack<T, V>(dst + (uint64_t)j * d.step, r[k]);
+      char *dst = tdst + (uint64_t)(base + cw + k * cpw) * UB + (uint64_t)m0 * d.step;
+      for (int j = m0; j < m1; j++, dst += d.step) st_pack<T, V>(dst, r[k]);
     }
   }
 }
 
 template <class T, int OP, int ORDER, bool MM, int U>
-__device__ __forceinline__ void run_desc_tile(const BDesc &d, uint32_t di, uint32_t lt,
-                                              const BPlan &p, uint32_t *stk) {
+__device__ __forceinline__ void run_one(const BTile &d, const BPlan &p, uint32_t *stk) {
   constexpr int V = sizeof(T) >= 16 ? 1 : (int)(16 / sizeof(T));
-  const uint64_t nvt = d.vec ? (d.npacks + d.TP - 1) / d.TP : 0;
-  if (d.vec && lt < nvt) {
-    const uint64_t pb = (uint64_t)lt * d.TP;
-    const uint64_t c = d.npacks - pb < (uint64_t)d.TP ? d.npacks - pb : (uint64_t)d.TP;
-    if constexpr (U > 1) run_tile_multi<T, OP, ORDER, MM, V, U>(d, di, pb, c, p);
-    else run_tile<T, OP, ORDER, MM, V>(d, di, pb, c, p, stk);
-  } else {
-    uint64_t eb, ec;
-    if (d.vec) { /* the < V elements after the packs */
-      eb = d.npacks * V;
-      ec = d.N - eb;
-    } else {
-      eb = (uint64_t)lt * d.TP;
-      ec = d.N - eb < (uint64_t)d.TP ? d.N - eb : (uint64_t)d.TP;
-    }
-    run_tile<T, OP, ORDER, MM, 1>(d, di, eb, ec, p, stk);
+  if (d.vec) {
+    if constexpr (U > 1) run_tile_multi<T, OP, ORDER, MM, V, U>(d, 0, d.cnt, p);
+    else run_tile<T, OP, ORDER, MM, V>(d, 0, d.cnt, p, stk);
+    if (d.tail == 0) return;
+  }
+  if constexpr (U > 1 && ORDER != ORD_CHAIN)
+    run_tile_multi<T, OP, ORDER, MM, 1, U>(d, (uint64_t)d.cnt * V, d.tail, p);
+  else
+    run_tile<T, OP, ORDER, MM, 1>(d, d.vec ? (uint64_t)d.cnt * V : 0, d.vec ? d.tail : d.cnt, p,
+                                  stk);
+}
+
+#define B200_CHAIN_KIDS(DS, T_, OP_, MM_)                                                     \
+  case kid_of(DS, OP_, ORD_CHAIN, 0): run_one<T_, OP_, ORD_CHAIN, MM_, 1>(t, p, nullptr); break; \
+  case kid_of(DS, OP_, ORD_CHAIN, 1): run_one<T_, OP_, ORD_CHAIN, MM_, 2>(t, p, nullptr); break; \
+  case kid_of(DS, OP_, ORD_CHAIN, 2): run_one<T_, OP_, ORD_CHAIN, MM_, 4>(t, p, nullptr); break;
+/* the ops whose bits do not depend on signedness run on the unsigned type
+ * (dslot_of maps both signs to one slot for them) */
+#define B200_WORD_KIDS(DS, U_)                                                                \
+  B200_CHAIN_KIDS(DS, U_, B200SHM_AND, false)                                                 \
+  B200_CHAIN_KIDS(DS, U_, B200SHM_OR, false)                                                  \
+  B200_CHAIN_KIDS(DS, U_, B200SHM_XOR, false)                                                 \
+  B200_CHAIN_KIDS(DS, U_, B200SHM_SUM, false)                                                 \
+  B200_CHAIN_KIDS(DS, U_, B200SHM_PROD, false)
+#define B200_ORDER_KIDS(DS, T_, MM_)                                                          \
+  B200_CHAIN_KIDS(DS, T_, B200SHM_MIN, MM_)                                                   \
+  B200_CHAIN_KIDS(DS, T_, B200SHM_MAX, MM_)
+
+#define B200_SMALL_KID(DS, F_, OP_)                                                           \
+  case kid_of(DS, OP_, ORD_BUTTERFLY, 1): run_one<F_, OP_, ORD_BUTTERFLY, false, 2>(t, p, nullptr); break;
+
+/* The order-free reductions, the left folds of the linear order, and the
+ * butterflies of small teams (at most two leaves per lane): no stack, 64
+ * registers, 4 CTAs per SM.  What bounds them is loads in flight, so the
+ * registers are kept down: a pointer per lane stepped from member to
+ * member, one register for a column's operand classes.  One CTA per tile
+ * (each starts with a 48-byte record of all it needs): CTAs start and end
+ * on their own, so no tile waits for a counter, a barrier, or the launch of
+ * another type.  Against one persistent launch per (type, op, order) --
+ * 62 of them in turn on four streams, 2 CTAs per SM at 128 registers, tiles
+ * of 1024 packs whatever the team -- the two launches here took 2048
+ * reductions over 256 teams (2.08 GB) from 800 to 385 us (2.60 to 5.39
+ * TB/s) and 97 reductions over 40 teams from 127 to 24 us.  With 3 CTAs per
+ * SM (80 registers) the 2048 ran in 413 us.  A batch of one int32 SUM shape
+ * runs at 6.0-6.4 TB/s for teams of 2 to 64. */
+__global__ void __launch_bounds__(kBatchThreads, 4) k_batch_chains(const BPlan p) {
+  const BTile t = p.tiles[blockIdx.x];
+  switch (t.kid) {
+    B200_WORD_KIDS(DS_U32, uint32_t)
+    B200_WORD_KIDS(DS_U64, uint64_t)
+    B200_ORDER_KIDS(DS_I32, int32_t, false)
+    B200_ORDER_KIDS(DS_U32, uint32_t, false)
+    B200_ORDER_KIDS(DS_I64, int64_t, false)
+    B200_ORDER_KIDS(DS_U64, uint64_t, false)
+    B200_ORDER_KIDS(DS_F32, float, true)
+    B200_ORDER_KIDS(DS_F64, double, true)
+    B200_CHAIN_KIDS(DS_F32, float, B200SHM_SUM, false)
+    B200_CHAIN_KIDS(DS_F32, float, B200SHM_PROD, false)
+    B200_CHAIN_KIDS(DS_F64, double, B200SHM_SUM, false)
+    B200_CHAIN_KIDS(DS_F64, double, B200SHM_PROD, false)
+    B200_SMALL_KID(DS_F32, float, B200SHM_SUM)
+    B200_SMALL_KID(DS_F32, float, B200SHM_PROD)
+    B200_SMALL_KID(DS_F64, double, B200SHM_SUM)
+    B200_SMALL_KID(DS_F64, double, B200SHM_PROD)
   }
 }
 
-/* One (type, op, order) group of a batch: descriptors [d0, d0+nd) of the
- * plan (sorted by group), tiles taken from the group's counter. */
-template <class T, int OP, int ORDER, bool MM, int U>
-__global__ void __launch_bounds__(kBatchThreads, 2) k_batch_group(const BPlan p, uint32_t d0,
-                                                               uint32_t nd, unsigned *counter) {
-  __shared__ unsigned s_tile;
-  /* 16-byte packs: 4 words per level per thread (chains keep no stack) */
-  __shared__ uint32_t s_stk[ORDER == ORD_CHAIN ? 1 : kBatchStackLevels * 4 * kBatchThreads];
-  const uint32_t base = p.prefix[d0], total = p.prefix[d0 + nd] - base;
-  /* A tile's descriptor comes from the plan's tile map in one load, not
-   * from a binary search over the group's descriptors. */
-  for (;;) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(counter, 1u);
-    __syncthreads();
-    const unsigned t = s_tile;
-    __syncthreads();
-    if (t >= total) return;
-    const uint2 m = p.tile_map[base + t];
-    const BDesc d = p.d[m.x];
-    run_desc_tile<T, OP, ORDER, MM, U>(d, m.x, m.y, p, s_stk);
+#define B200_TREE_KIDS(DS, F_, OP_)                                                           \
+  case kid_of(DS, OP_, ORD_BINOMIAL, 0): run_one<F_, OP_, ORD_BINOMIAL, false, 1>(t, p, s_stk); break; \
+  case kid_of(DS, OP_, ORD_BUTTERFLY, 0): run_one<F_, OP_, ORD_BUTTERFLY, false, 1>(t, p, s_stk); break;
+
+/* The float trees with more than two leaves per lane (SUM/PROD in a
+ * binomial or butterfly order): 128 registers and 2 CTAs per SM.  Held to
+ * 80 registers (3 CTAs) they spill, and the 2048 reductions ran in 397 us
+ * against 385; at 64 registers with four leaves at a time, teams of 100 to
+ * 200 members lost 15-20 %. */
+__global__ void __launch_bounds__(kBatchThreads, 2) k_batch_trees(const BPlan p) {
+  /* 16-byte packs: 4 words per level per thread */
+  __shared__ uint32_t s_stk[kBatchStackLevels * 4 * kBatchThreads];
+  const BTile t = p.tiles[blockIdx.x];
+  switch (t.kid) {
+    B200_TREE_KIDS(DS_F32, float, B200SHM_SUM)
+    B200_TREE_KIDS(DS_F32, float, B200SHM_PROD)
+    B200_TREE_KIDS(DS_F64, double, B200SHM_SUM)
+    B200_TREE_KIDS(DS_F64, double, B200SHM_PROD)
   }
 }
 
@@ -481,11 +561,12 @@ __global__ void __launch_bounds__(256) k_batch_fix(const BPlan p) {
 }
 
 /* ---- host-side planning -------------------------------------------------- */
-int dslot_of(int dtype) {
+int dslot_of(int dtype, int op) {
+  const bool mm = op == B200SHM_MIN || op == B200SHM_MAX;
   switch (dtype) {
-  case B200SHM_I32: return DS_I32;
+  case B200SHM_I32: return mm ? DS_I32 : DS_U32;
   case B200SHM_U32: return DS_U32;
-  case B200SHM_I64: return DS_I64;
+  case B200SHM_I64: return mm ? DS_I64 : DS_U64;
   case B200SHM_U64: return DS_U64;
   case B200SHM_F32: return DS_F32;
   case B200SHM_F64: return DS_F64;
@@ -557,86 +638,69 @@ bool lanes_ok(const BDesc &d, int G) {
   return nleaves / G <= kBatchMaxLaneLeaves;
 }
 
-uint32_t tiles_of(const BDesc &d) {
-  if (d.vec) {
-    const uint64_t V = 16 / (uint64_t)esize_of(d);
-    const uint64_t t = (d.npacks + d.TP - 1) / d.TP;
-    return (uint32_t)(t + (d.N > d.npacks * V ? 1 : 0));
-  }
-  return (uint32_t)((d.N + d.TP - 1) / d.TP);
+/* Units (packs, or elements of an unaligned descriptor) of one tile: the
+ * plan's TP, less where the team has more than 8 members, so that a tile
+ * reads 128 bytes x TP (128 KiB as planned by default) whatever the team's
+ * size -- but at least one pass of the CTA over its columns.  A tile of TP
+ * units of a 256-member team would be one CTA's work for 150 us, the time
+ * the whole of a small batch takes.  Budgets of 32 / 64 / 128 / 256 bytes x
+ * TP ran 2048 reductions over 256 teams within 2 % of each other; more
+ * lanes per column for teams above 64 members, to cut the pass itself,
+ * lost 6 % (shorter runs of each member). */
+uint64_t tile_units(const BDesc &d) {
+  const uint64_t pass = (uint64_t)kBatchThreads / d.G * d.U;
+  const uint64_t unit = d.vec ? 16 : esize_of(d);
+  uint64_t u = (uint64_t)d.TP * 128 / (unit * (uint64_t)d.P);
+  if (u > (uint64_t)d.TP) u = d.TP;
+  u = u / pass * pass;
+  return u < pass ? pass : u;
 }
+inline bool is_tree(const BDesc &d) { return order_of(d) != ORD_CHAIN && d.U == 1; }
 
-/* An uploaded plan: descriptors sorted by (type, op, order) group, tile
- * prefix sums, one tile counter per group. */
-struct Group {
-  int kid;
-  uint32_t d0, nd, tiles;
-  int grid;
-};
 struct Batch {
-  std::vector<BDesc> hd;
-  std::vector<uint32_t> hp;
-  std::vector<Group> groups;
+  std::vector<BDesc> hd;                     /* chains first, then trees */
   std::vector<b200shm_reduce_desc> fallback; /* run as separate launches */
+  uint32_t ntiles[2] = {0, 0};               /* of the chains, of the trees */
   BDesc *dd = nullptr;
-  uint32_t *dp = nullptr;
-  uint2 *dmap = nullptr; /* tile map (BPlan::tile_map) */
-  unsigned *dcount = nullptr;
+  BTile *dt = nullptr;
   bool any_mm = false;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   unsigned graph_launches = 0; /* kernels one replay of `exec` runs */
-  /* side streams the groups are spread over, so that one group's tail
-   * overlaps the next group's start (forked from and joined back into the
-   * caller's stream with events; inside a capture they become branches) */
-  std::vector<cudaStream_t> side;
-  std::vector<cudaEvent_t> ev; /* ev[0] = fork, ev[1 + k] = join of side[k] */
-  cudaEvent_t done = nullptr;  /* recorded after each run on the caller's stream */
+  /* the trees run beside the chains on a side stream (forked from and
+   * joined back into the caller's stream with events; inside a capture it
+   * becomes a branch) */
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaEvent_t done = nullptr; /* recorded after each run on the caller's stream */
 };
-
-constexpr int kBatchSideStreams = 4;
 
 /* Free a plan whose runs have completed (ordered on the library stream). */
 void release(Batch &b) {
-  for (cudaStream_t x : b.side) cudaStreamDestroy(x);
-  for (cudaEvent_t e : b.ev) cudaEventDestroy(e);
-  if (b.done) cudaEventDestroy(b.done);
-  b.done = nullptr;
-  b.side.clear();
-  b.ev.clear();
+  if (b.side) cudaStreamDestroy(b.side);
+  for (cudaEvent_t *e : {&b.fork, &b.join, &b.done}) {
+    if (*e) cudaEventDestroy(*e);
+    *e = nullptr;
+  }
+  b.side = nullptr;
   if (b.dd) cudaFreeAsync(b.dd, st().stream);
-  if (b.dp) cudaFreeAsync(b.dp, st().stream);
-  if (b.dmap) cudaFreeAsync(b.dmap, st().stream);
-  if (b.dcount) cudaFreeAsync(b.dcount, st().stream);
+  if (b.dt) cudaFreeAsync(b.dt, st().stream);
   b.dd = nullptr;
-  b.dp = nullptr;
-  b.dmap = nullptr;
-  b.dcount = nullptr;
+  b.dt = nullptr;
 }
 
 int make_side(Batch &b) {
-  const int k = (int)std::min<size_t>(b.groups.size(), kBatchSideStreams);
-  if (k < 2) return B200SHM_OK;
-  for (int i = 0; i < k; i++) {
-    cudaStream_t x;
-    B200_CK(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
-    b.side.push_back(x);
-  }
-  for (int i = 0; i <= k; i++) {
-    cudaEvent_t e;
-    B200_CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    b.ev.push_back(e);
-  }
+  if (!b.ntiles[0] || !b.ntiles[1]) return B200SHM_OK;
+  B200_CK(cudaStreamCreateWithFlags(&b.side, cudaStreamNonBlocking));
+  B200_CK(cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming));
+  B200_CK(cudaEventCreateWithFlags(&b.join, cudaEventDisableTiming));
   return B200SHM_OK;
 }
 
 BPlan plan_of(const Batch &b) {
   BPlan p;
   p.d = b.dd;
-  p.prefix = b.dp;
-  p.tile_map = b.dmap;
-  p.ndesc = (uint32_t)b.hd.size();
-  p.total = b.hp.empty() ? 0 : b.hp.back();
+  p.tiles = b.dt;
   p.fix_list = st().fix_list;
   p.fix_count = st().fix_count;
   p.fix_cap = st().fix_cap;
@@ -644,82 +708,28 @@ BPlan plan_of(const Batch &b) {
   return p;
 }
 
-/* the group kernel of a kid, and its resident CTAs per SM */
-typedef void (*GroupKernel)(const BPlan, uint32_t, uint32_t, unsigned *);
-template <class T, int OP, int ORDER, bool MM, int U>
-GroupKernel gk() {
-  return k_batch_group<T, OP, ORDER, MM, U>;
-}
-#define B200_CHAIN_KIDS(DS, T_, OP_, MM_)                                               \
-  case kid_of(DS, OP_, ORD_CHAIN, 0): return gk<T_, OP_, ORD_CHAIN, MM_, 1>();          \
-  case kid_of(DS, OP_, ORD_CHAIN, 1): return gk<T_, OP_, ORD_CHAIN, MM_, 2>();          \
-  case kid_of(DS, OP_, ORD_CHAIN, 2): return gk<T_, OP_, ORD_CHAIN, MM_, 4>();
-#define B200_INT_KIDS(DS, S_, U_)                                                       \
-  B200_CHAIN_KIDS(DS, U_, B200SHM_AND, false)                                           \
-  B200_CHAIN_KIDS(DS, U_, B200SHM_OR, false)                                            \
-  B200_CHAIN_KIDS(DS, U_, B200SHM_XOR, false)                                           \
-  B200_CHAIN_KIDS(DS, S_, B200SHM_MIN, false)                                           \
-  B200_CHAIN_KIDS(DS, S_, B200SHM_MAX, false)                                           \
-  B200_CHAIN_KIDS(DS, U_, B200SHM_SUM, false)                                           \
-  B200_CHAIN_KIDS(DS, U_, B200SHM_PROD, false)
-#define B200_TREE_KIDS(DS, F_, OP_)                                                     \
-  case kid_of(DS, OP_, ORD_BINOMIAL, 0): return gk<F_, OP_, ORD_BINOMIAL, false, 1>();  \
-  case kid_of(DS, OP_, ORD_BUTTERFLY, 0): return gk<F_, OP_, ORD_BUTTERFLY, false, 1>();\
-  case kid_of(DS, OP_, ORD_BUTTERFLY, 1): return gk<F_, OP_, ORD_BUTTERFLY, false, 2>();
-#define B200_FLT_KIDS(DS, F_)                                                           \
-  B200_CHAIN_KIDS(DS, F_, B200SHM_MIN, true)                                            \
-  B200_CHAIN_KIDS(DS, F_, B200SHM_MAX, true)                                            \
-  B200_CHAIN_KIDS(DS, F_, B200SHM_SUM, false)                                           \
-  B200_CHAIN_KIDS(DS, F_, B200SHM_PROD, false)                                          \
-  B200_TREE_KIDS(DS, F_, B200SHM_SUM)                                                   \
-  B200_TREE_KIDS(DS, F_, B200SHM_PROD)
-GroupKernel group_kernel(int kid) {
-  switch (kid) {
-    B200_INT_KIDS(DS_I32, int32_t, uint32_t)
-    B200_INT_KIDS(DS_U32, uint32_t, uint32_t)
-    B200_INT_KIDS(DS_I64, int64_t, uint64_t)
-    B200_INT_KIDS(DS_U64, uint64_t, uint64_t)
-    B200_FLT_KIDS(DS_F32, float)
-    B200_FLT_KIDS(DS_F64, double)
-  default: return nullptr;
-  }
-}
-int resident_ctas(int kid) {
-  static std::mutex mu;
-  static std::map<int, int> occ;
-  std::lock_guard<std::mutex> lk(mu);
-  auto it = occ.find(kid);
-  if (it != occ.end()) return it->second;
-  int o = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, group_kernel(kid), kBatchThreads, 0) !=
-          cudaSuccess ||
-      o < 1)
-    o = 1;
-  occ[kid] = o;
-  return o;
-}
-
 int enqueue(const Batch &b, cudaStream_t s) {
   if (!b.hd.empty()) {
-    B200_CK(cudaMemsetAsync(b.dcount, 0, b.groups.size() * sizeof(unsigned), s));
     if (b.any_mm) B200_CK(cudaMemsetAsync(st().fix_count, 0, sizeof(unsigned long long), s));
-    const BPlan p = plan_of(b);
-    const size_t ns = b.side.size();
-    if (ns) {
-      B200_CK(cudaEventRecord(b.ev[0], s));
-      for (size_t k = 0; k < ns; k++) B200_CK(cudaStreamWaitEvent(b.side[k], b.ev[0], 0));
+    BPlan p = plan_of(b);
+    cudaStream_t ts = b.side ? b.side : s;
+    if (b.side) {
+      B200_CK(cudaEventRecord(b.fork, s));
+      B200_CK(cudaStreamWaitEvent(b.side, b.fork, 0));
     }
-    for (size_t gi = 0; gi < b.groups.size(); gi++) {
-      const Group &g = b.groups[gi];
-      cudaStream_t gs = ns ? b.side[gi % ns] : s;
-      group_kernel(g.kid)<<<g.grid, kBatchThreads, 0, gs>>>(p, g.d0, g.nd, b.dcount + gi);
+    if (b.ntiles[1]) { /* the trees' tiles take longer: they start first */
+      BPlan pt = p;
+      pt.tiles += b.ntiles[0];
+      k_batch_trees<<<b.ntiles[1], kBatchThreads, 0, ts>>>(pt);
       count_launch();
     }
-    if (ns) {
-      for (size_t k = 0; k < ns; k++) {
-        B200_CK(cudaEventRecord(b.ev[1 + k], b.side[k]));
-        B200_CK(cudaStreamWaitEvent(s, b.ev[1 + k], 0));
-      }
+    if (b.ntiles[0]) {
+      k_batch_chains<<<b.ntiles[0], kBatchThreads, 0, s>>>(p);
+      count_launch();
+    }
+    if (b.side) {
+      B200_CK(cudaEventRecord(b.join, b.side));
+      B200_CK(cudaStreamWaitEvent(s, b.join, 0));
     }
     if (b.any_mm) {
       k_batch_fix<<<2 * st().sm_count, 256, 0, s>>>(p);
@@ -734,44 +744,59 @@ int enqueue(const Batch &b, cudaStream_t s) {
   return B200SHM_OK;
 }
 
-/* Sort by group (stable), build prefix sums and groups, upload. */
+/* Bytes one tile of d reads: what it costs its CTA. */
+uint64_t tile_cost(const BDesc &d) {
+  const uint64_t units = d.vec ? d.npacks : d.N;
+  return std::min(tile_units(d), units) * (d.vec ? 16 : esize_of(d)) * (uint64_t)d.P;
+}
+
+/* Sort the descriptors (chains, then trees; the largest tiles first, by
+ * powers of two, so that the last CTAs to run are short; tiles of a size by
+ * type and op, so that CTAs that run together share their instructions:
+ * 385 us, 400 without), cut them into tiles, upload. */
 int upload(Batch &b) {
   const size_t nd = b.hd.size();
   if (nd == 0) return B200SHM_OK;
-  std::stable_sort(b.hd.begin(), b.hd.end(),
-                   [](const BDesc &x, const BDesc &y) { return x.kid < y.kid; });
-  b.hp.assign(nd + 1, 0);
-  for (size_t i = 0; i < nd; i++) b.hp[i + 1] = b.hp[i] + tiles_of(b.hd[i]);
-  b.groups.clear();
-  for (size_t i = 0; i < nd;) {
-    size_t j = i;
-    while (j < nd && b.hd[j].kid == b.hd[i].kid) j++;
-    Group g;
-    g.kid = b.hd[i].kid;
-    g.d0 = (uint32_t)i;
-    g.nd = (uint32_t)(j - i);
-    g.tiles = b.hp[j] - b.hp[i];
-    const uint64_t cap = (uint64_t)st().sm_count * (uint64_t)resident_ctas(g.kid);
-    g.grid = (int)(g.tiles < cap ? (g.tiles ? g.tiles : 1) : cap);
-    b.groups.push_back(g);
-    i = j;
+  std::stable_sort(b.hd.begin(), b.hd.end(), [](const BDesc &x, const BDesc &y) {
+    if (is_tree(x) != is_tree(y)) return is_tree(y);
+    const int cx = log2_floor(tile_cost(x)), cy = log2_floor(tile_cost(y));
+    return cx != cy ? cx > cy : x.kid < y.kid;
+  });
+  std::vector<BTile> tiles;
+  b.ntiles[0] = b.ntiles[1] = 0;
+  for (size_t i = 0; i < nd; i++) {
+    const BDesc &d = b.hd[i];
+    const uint64_t es = esize_of(d), V = d.vec ? 16 / es : 1;
+    const uint64_t units = d.vec ? d.npacks : d.N, per = tile_units(d);
+    const uint64_t nt = units ? (units + per - 1) / per : 1; /* no pack at all: a tail */
+    for (uint64_t t = 0; t < nt; t++) {
+      BTile x;
+      const uint64_t u0 = t * per;
+      x.e0 = u0 * V;
+      x.src = d.src + x.e0 * es;
+      x.dst = d.dst + x.e0 * es;
+      x.step = d.step;
+      x.di = (uint32_t)i;
+      x.cnt = (uint32_t)std::min(per, units - u0);
+      x.P = (uint16_t)d.P;
+      x.kid = (uint16_t)d.kid;
+      x.G = (uint8_t)d.G;
+      x.vec = (uint8_t)d.vec;
+      x.tail = (uint8_t)(d.vec && t == nt - 1 ? d.N - units * V : 0);
+      x.pad = 0;
+      tiles.push_back(x);
+    }
+    b.ntiles[is_tree(d)] += (uint32_t)nt;
   }
+  if (tiles.size() > 0x7fffffffull) return fail(B200SHM_ERR_ARG, "batch_create: too many tiles");
   /* stream-ordered allocations: no device-wide synchronisation, so a
    * running serving loop does not hold them up */
   cudaStream_t ls = st().stream;
   B200_CK(cudaMallocAsync((void **)&b.dd, nd * sizeof(BDesc), ls));
-  B200_CK(cudaMallocAsync((void **)&b.dp, (nd + 1) * sizeof(uint32_t), ls));
-  const uint32_t ntiles = b.hp[nd];
-  std::vector<uint2> map(ntiles ? ntiles : 1);
-  for (size_t i = 0; i < nd; i++)
-    for (uint32_t t = b.hp[i]; t < b.hp[i + 1]; t++) map[t] = make_uint2((unsigned)i, t - b.hp[i]);
-  B200_CK(cudaMallocAsync((void **)&b.dmap, map.size() * sizeof(uint2), ls));
-  B200_CK(cudaMemcpyAsync(b.dmap, map.data(), map.size() * sizeof(uint2), cudaMemcpyHostToDevice,
-                          ls));
-  B200_CK(cudaMallocAsync((void **)&b.dcount, b.groups.size() * sizeof(unsigned), ls));
+  B200_CK(cudaMallocAsync((void **)&b.dt, tiles.size() * sizeof(BTile), ls));
   B200_CK(cudaMemcpyAsync(b.dd, b.hd.data(), nd * sizeof(BDesc), cudaMemcpyHostToDevice, ls));
-  B200_CK(cudaMemcpyAsync(b.dp, b.hp.data(), (nd + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice,
-                          ls));
+  B200_CK(cudaMemcpyAsync(b.dt, tiles.data(), tiles.size() * sizeof(BTile),
+                          cudaMemcpyHostToDevice, ls));
   B200_CK(cudaStreamSynchronize(ls)); /* the plan is then usable on any stream */
   return B200SHM_OK;
 }
@@ -836,7 +861,7 @@ float time_batch(Batch &b, const std::vector<BDesc> &base, cudaStream_t s) {
  * (cached choices, else the heuristic); then, for the shape classes that
  * carry the most bytes and have no cached choice yet, one class at a time,
  * give every descriptor of the class each other (lanes per column, tile)
- * and time the WHOLE batch -- its groups overlapping on the side streams,
+ * and time the WHOLE batch -- its launches side by side,
  * as a run does -- keeping a change only when the batch got more than 1 %
  * faster.  The choices go to the per-process cache, which later batches
  * start from.  (Timing a shape class alone, where launch overhead
@@ -1003,7 +1028,7 @@ int b200shm_batch_create(b200shm_reduce_desc *descs, uint64_t n, int flags,
     if (rc)
       return bail(fail(rc, "batch descriptor %llu: %s", (unsigned long long)i,
                        b200shm_last_error()));
-    const int ds = dslot_of(x.dtype);
+    const int ds = dslot_of(x.dtype, x.op);
     const bool is_int = x.dtype <= B200SHM_U64;
     const bool mm = x.op == B200SHM_MIN || x.op == B200SHM_MAX;
     int order = ORD_CHAIN;
