@@ -1001,8 +1001,8 @@ def run_batch(args, world, rank, local):
             "batched": {"ms": round(b_ms, 4), "ops_per_s": round(len(items) / (b_ms / 1e3), 1),
                         "gbs": round(total_bytes / (b_ms / 1e3) / 1e9, 1),
                         "frac_of_hbm": round(total_bytes / (b_ms / 1e3) / 1e9 / peak, 4),
-                        "form": "CUDA graph: one persistent kernel per (type, op, order) group "
-                                "on 4 side streams + MIN/MAX replay",
+                        "form": "CUDA graph: the tiles of all reductions in two launches "
+                                "side by side + MIN/MAX replay",
                         "plan_seconds": round(plan_s, 2), "autotune": args.batch_tune,
                         "heuristic_plan_ms": round(h_ms, 4),
                         "tuned_vs_heuristic": round(h_ms / b_ms, 3),

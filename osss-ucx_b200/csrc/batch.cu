@@ -89,27 +89,6 @@ struct BPlan {
   int *status;
 };
 
-/* The member step, as a value the compiler cannot multiply ahead: eight
- * precomputed multiples of it cost a lane 16 registers, eight additions
- * cost next to nothing beside eight loads. */
-__device__ __forceinline__ uint64_t opaque(uint64_t v) {
-  asm volatile("" : "+l"(v));
-  return v;
-}
-
-/* A column's operand classes (fclass, 3 bits an element) in one register. */
-template <class PK>
-__device__ __forceinline__ unsigned pack_class(const PK &v) {
-  unsigned c = 0;
-#pragma unroll
-  for (int i = 0; i < (int)(sizeof(v.x) / sizeof(v.x[0])); i++) c |= fclass(v.x[i]) << (3 * i);
-  return c;
-}
-/* some element saw a NaN, or zeros of both signs */
-__device__ __forceinline__ bool pack_ambiguous(unsigned c) {
-  return ((c & 01111u) | ((c >> 1) & (c >> 2) & 01111u)) != 0;
-}
-
 /* A lane's stack of complete subtrees lives in shared memory, one 32-bit
  * word per thread per row ([level][word][thread]), so that a warp's
  * accesses fall in 32 distinct banks. */
@@ -157,7 +136,8 @@ __device__ __forceinline__ void run_tile(const BTile &d, uint64_t at, uint32_t c
   };
   const int m0 = member_of(l0), m1 = member_of(l1);
   auto comb = [](const PK &lo, const PK &hi) {
-    if constexpr (ORDER == ORD_BINOMIAL) return papply<OP>(hi, lo);
+    if constexpr (MM) return mm_combine<OP>(lo, hi);
+    else if constexpr (ORDER == ORD_BINOMIAL) return papply<OP>(hi, lo);
     else return papply<OP>(lo, hi);
   };
   for (uint32_t base = warp * cpw; base < cnt; base += nw * cpw) {
@@ -171,8 +151,8 @@ __device__ __forceinline__ void run_tile(const BTile &d, uint64_t at, uint32_t c
       if constexpr (ORDER == ORD_CHAIN) {
         const char *q = src + (uint64_t)m0 * d.step;
         r = ld_pack<T, V>(q);
-        if constexpr (MM) cls = pack_class(r);
-        for (int j = m0 + 1; j < m1; j += 8) {
+        int j = m0 + 1;
+        do { /* once at least: a MIN/MAX lane looks at its first operand below the loads */
           PK x[8];
           const uint64_t step = opaque(d.step);
 #pragma unroll
@@ -180,13 +160,16 @@ __device__ __forceinline__ void run_tile(const BTile &d, uint64_t at, uint32_t c
             q += step;
             if (j + u < m1) x[u] = ld_pack<T, V>(q);
           }
+          if constexpr (MM)
+            if (j == m0 + 1) cls = mm_flags<OP>(r);
 #pragma unroll
           for (int u = 0; u < 8; u++)
             if (j + u < m1) {
-              r = papply<OP>(r, x[u]);
-              if constexpr (MM) cls |= pack_class(x[u]);
+              r = comb(r, x[u]);
+              if constexpr (MM) cls |= mm_flags<OP>(x[u]);
             }
-        }
+          j += 8;
+        } while (j < m1);
       } else {
         /* The lane's leaves are taken KB at a time: their own members and
          * (for a butterfly over a non-power-of-two team) extra members
@@ -274,7 +257,7 @@ __device__ __forceinline__ void run_tile(const BTile &d, uint64_t at, uint32_t c
     }
     if (!live) continue;
     if constexpr (MM) {
-      if (pack_ambiguous(cls)) { /* deferred: (descriptor, element) pairs, dests untouched */
+      if (mm_ambiguous<OP>(r, cls)) { /* deferred: (descriptor, element) pairs, dests untouched */
         if (g == 0) {
           const unsigned long long slot = atomicAdd(p.fix_count, (unsigned long long)V);
           for (int i = 0; i < V; i++) {
@@ -316,7 +299,10 @@ __device__ __forceinline__ void run_tile_multi(const BTile &d, uint64_t at, uint
   const char *tsrc = d.src + at * sizeof(T);
   char *tdst = d.dst + at * sizeof(T);
   const int m0 = member_of(l0), m1 = member_of(l1);
-  auto comb = [](const PK &lo, const PK &hi) { return papply<OP>(lo, hi); };
+  auto comb = [](const PK &lo, const PK &hi) {
+    if constexpr (MM) return mm_combine<OP>(lo, hi);
+    else return papply<OP>(lo, hi);
+  };
   for (uint32_t base = warp * cpw * U; base < cnt; base += nw * cpw * U) {
     PK r[U];
     unsigned cls[U];
@@ -336,11 +322,9 @@ __device__ __forceinline__ void run_tile_multi(const BTile &d, uint64_t at, uint
       const char *q = src0 + (uint64_t)m0 * d.step;
 #pragma unroll
       for (int k = 0; k < U; k++)
-        if (live[k]) {
-          r[k] = ld_pack<T, V>(q + k * gap);
-          if constexpr (MM) cls[k] = pack_class(r[k]);
-        }
-      for (int j = m0 + 1; j < m1; j += MB) {
+        if (live[k]) r[k] = ld_pack<T, V>(q + k * gap);
+      int j = m0 + 1;
+      do {
         PK x[U][MB];
         const uint64_t step = opaque(d.step);
 #pragma unroll
@@ -350,15 +334,22 @@ __device__ __forceinline__ void run_tile_multi(const BTile &d, uint64_t at, uint
           for (int k = 0; k < U; k++)
             if (live[k] && j + u < m1) x[k][u] = ld_pack<T, V>(q + k * gap);
         }
+        if constexpr (MM) {
+          if (j == m0 + 1) {
+#pragma unroll
+            for (int k = 0; k < U; k++) cls[k] = mm_flags<OP>(r[k]);
+          }
+        }
 #pragma unroll
         for (int k = 0; k < U; k++)
 #pragma unroll
           for (int u = 0; u < MB; u++)
             if (live[k] && j + u < m1) {
-              r[k] = papply<OP>(r[k], x[k][u]);
-              if constexpr (MM) cls[k] |= pack_class(x[k][u]);
+              r[k] = comb(r[k], x[k][u]);
+              if constexpr (MM) cls[k] |= mm_flags<OP>(x[k][u]);
             }
-      }
+        j += MB;
+      } while (j < m1);
     } else { /* butterfly, l1 - l0 in {1, 2} leaves per lane */
       const int n = l1 - l0;
       PK x[U][2], e[U][2];
@@ -400,7 +391,7 @@ __device__ __forceinline__ void run_tile_multi(const BTile &d, uint64_t at, uint
     for (int k = 0; k < U; k++) {
       if (!live[k]) continue;
       if constexpr (MM) {
-        if (pack_ambiguous(cls[k])) { /* deferred: (descriptor, element) pairs, dests untouched */
+        if (mm_ambiguous<OP>(r[k], cls[k])) { /* deferred: (descriptor, element) pairs, dests untouched */
           if (g == 0) {
             const unsigned long long slot = atomicAdd(p.fix_count, (unsigned long long)V);
             const uint64_t e0 = at + (uint64_t)(base + cw + k * cpw) * V;

@@ -64,8 +64,9 @@ static RArgs reduce_args(const char *src, char *dst, uint64_t sstep, uint64_t ds
   a.dst = dst;
   a.sstep = sstep;
   a.dstep = dstep;
-  a.e_begin = 0;
+  a.head = a.nedge = 0;
   a.nvec = 0;
+  a.lgG = 0;
   a.N = nelems;
   a.g_off = 0;
   a.g_n = nelems;
@@ -79,7 +80,7 @@ static RArgs reduce_args(const char *src, char *dst, uint64_t sstep, uint64_t ds
   return a;
 }
 
-static int reduce_dispatch(int op, int dtype, const RArgs &a, bool aligned, cudaStream_t s);
+static int reduce_dispatch(int op, int dtype, const RArgs &a, cudaStream_t s);
 
 int reduce_launch(int op, int dtype, int algo, int pe_start, int pe_stride, int pe_size,
                   uint64_t dest_off, uint64_t src_off, uint64_t nelems, cudaStream_t s) {
@@ -102,8 +103,7 @@ int reduce_launch(int op, int dtype, int algo, int pe_start, int pe_stride, int 
   a.fix_done = st().call_fix + 1;
   a.fix_cap = st().fix_cap;
   a.status = st().d_status;
-  const bool aligned = ((src_off | dest_off | m.step) & 15u) == 0;
-  return reduce_dispatch(op, dtype, a, aligned, s);
+  return reduce_dispatch(op, dtype, a, s);
 }
 
 /* Elements [e0, e0 + count) of a reduction of nelems elements (validated by
@@ -124,24 +124,23 @@ int reduce_range_launch(int op, int dtype, int algo, int pe_start, int pe_stride
   a.fix_done = st().call_fix + 1;
   a.fix_cap = st().fix_cap;
   a.status = st().d_status;
-  const bool aligned = (((src_off + e0 * es) | (dest_off + e0 * es) | m.step) & 15u) == 0;
-  return reduce_dispatch(op, dtype, a, aligned, s);
+  return reduce_dispatch(op, dtype, a, s);
 }
 
-static int reduce_dispatch(int op, int dtype, const RArgs &a, bool aligned, cudaStream_t s) {
+static int reduce_dispatch(int op, int dtype, const RArgs &a, cudaStream_t s) {
   switch (dtype) {
-  case B200SHM_F32: return reduce_dispatch_f32(op, a, aligned, s);
-  case B200SHM_F64: return reduce_dispatch_f64(op, a, aligned, s);
+  case B200SHM_F32: return reduce_dispatch_f32(op, a, s);
+  case B200SHM_F64: return reduce_dispatch_f64(op, a, s);
   case B200SHM_F80:
     switch (op) {
-    case B200SHM_MIN: return reduce_dispatch_f80_min(a, aligned, s);
-    case B200SHM_MAX: return reduce_dispatch_f80_max(a, aligned, s);
-    case B200SHM_SUM: return reduce_dispatch_f80_sum(a, aligned, s);
-    default: return reduce_dispatch_f80_prod(a, aligned, s);
+    case B200SHM_MIN: return reduce_dispatch_f80_min(a, s);
+    case B200SHM_MAX: return reduce_dispatch_f80_max(a, s);
+    case B200SHM_SUM: return reduce_dispatch_f80_sum(a, s);
+    default: return reduce_dispatch_f80_prod(a, s);
     }
-  case B200SHM_C32: return reduce_dispatch_c32(op, a, aligned, s);
-  case B200SHM_C64: return reduce_dispatch_c64(op, a, aligned, s);
-  default: return reduce_dispatch_int(op, dtype, a, aligned, s);
+  case B200SHM_C32: return reduce_dispatch_c32(op, a, s);
+  case B200SHM_C64: return reduce_dispatch_c64(op, a, s);
+  default: return reduce_dispatch_int(op, dtype, a, s);
   }
 }
 
@@ -368,8 +367,7 @@ extern "C" int b200shm_reduce_noalloc(int op, int dtype, int algo, int npes, voi
   /* the scratch keeps the previous call's contents: clear the counter, the
    * status word and the replay's exit counter first */
   B200_CK(cudaMemsetAsync(scratch, 0, 3 * sizeof(unsigned long long), s));
-  const bool aligned = (((uintptr_t)dest | (uintptr_t)source | dest_stride | source_stride) & 15u) == 0;
-  if ((rc = reduce_dispatch(op, dtype, a, aligned, s))) return rc;
+  if ((rc = reduce_dispatch(op, dtype, a, s))) return rc;
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "b200shm_reduce_noalloc launch");
   e = cudaStreamSynchronize(s);

@@ -7,9 +7,9 @@
 
 namespace b200 {
 
-int reduce_dispatch_c64(int op, const RArgs &a, bool aligned, cudaStream_t s) {
-  return op == B200SHM_SUM ? run_cplx<cf64, B200SHM_SUM>(a, aligned, s)
-                           : run_cplx<cf64, B200SHM_PROD>(a, aligned, s);
+int reduce_dispatch_c64(int op, const RArgs &a, cudaStream_t s) {
+  return op == B200SHM_SUM ? run_cplx<cf64, B200SHM_SUM>(a, s)
+                           : run_cplx<cf64, B200SHM_PROD>(a, s);
 }
 
 }  // namespace b200

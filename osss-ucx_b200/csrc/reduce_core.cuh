@@ -248,6 +248,43 @@ __device__ __forceinline__ void st_pack(char *p, const Pack<T, V> &v) {
     memcpy(p, &v, sizeof(v));
   }
 }
+/* The member step, as a value the compiler cannot multiply ahead: eight
+ * precomputed multiples of it cost a lane 16 registers, eight additions
+ * cost next to nothing beside eight loads. */
+__device__ __forceinline__ uint64_t opaque(uint64_t v) {
+  asm volatile("" : "+l"(v));
+  return v;
+}
+
+/* a pack at any address: the widest accesses it allows */
+template <class T, int V>
+__device__ __forceinline__ Pack<T, V> ld_any(const char *p) {
+  typedef Pack<T, V> PK;
+  PK r;
+  if constexpr (sizeof(PK) == 16) {
+    uint32_t w[4];
+    ld16_any(p, w);
+    memcpy(&r, w, 16);
+  } else if (((uintptr_t)p & (sizeof(PK) - 1)) == 0) {
+    r = *(const PK *)p;
+  } else {
+    memcpy(&r, p, sizeof(PK));
+  }
+  return r;
+}
+template <class T, int V>
+__device__ __forceinline__ void st_any(char *p, const Pack<T, V> &v) {
+  typedef Pack<T, V> PK;
+  if constexpr (sizeof(PK) == 16) {
+    uint32_t w[4];
+    memcpy(w, &v, 16);
+    st16_any(p, w);
+  } else if (((uintptr_t)p & (sizeof(PK) - 1)) == 0) {
+    *(PK *)p = v;
+  } else {
+    memcpy(p, &v, sizeof(PK));
+  }
+}
 template <int OP, class T, int V>
 __device__ __forceinline__ Pack<T, V> papply(const Pack<T, V> &a, const Pack<T, V> &b) {
   Pack<T, V> r;
@@ -276,6 +313,88 @@ __device__ __forceinline__ unsigned fclass(const f80 &f) {
   return 0u;
 }
 __device__ __forceinline__ bool ambiguous(unsigned f) { return (f & 1u) || (f & 6u) == 6u; }
+/* A column's operand classes, 3 bits an element, in one register. */
+template <class PK>
+__device__ __forceinline__ unsigned pack_class(const PK &v) {
+  unsigned c = 0;
+#pragma unroll
+  for (int i = 0; i < (int)(sizeof(v.x) / sizeof(v.x[0])); i++) c |= fclass(v.x[i]) << (3 * i);
+  return c;
+}
+/* some element saw a NaN, or zeros of both signs */
+__device__ __forceinline__ bool pack_ambiguous(unsigned c) {
+  return ((c & 01111u) | ((c >> 1) & (c >> 2) & 01111u)) != 0;
+}
+
+/* Float MIN/MAX as the streaming kernels run it.  The combine is the
+ * hardware's max/min, in which +0 is above -0 (and a NaN operand gives NaN
+ * for float), so of the classes above only one zero has to be watched for:
+ * the result is order dependent when an operand was a NaN, or when the
+ * result is +0 (MAX) and a -0 went in, or -0 (MIN) and a +0 went in.  Any
+ * other result is the operands' one maximum, with one pattern of bits, in
+ * whatever order they combine.  Flags of a column: bit i, the other zero
+ * seen in element i; bit 8 + i, a NaN (double).  Three instructions an
+ * element (float) for ten with the classes.  Together with looking at a
+ * lane's first operand only below its first loads (which the classes had
+ * waited for one by one), f64 MAX over teams of 2, 16384 elements a
+ * reduction, in a batch: 5.09 -> 6.05 TB/s. */
+template <int OP, class T>
+__device__ __forceinline__ T mm_pick(T a, T b) {
+  T r;
+  if constexpr (std::is_same<T, float>::value) {
+    if constexpr (OP == B200SHM_MAX) asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    else asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  } else if constexpr (std::is_same<T, double>::value) {
+    if constexpr (OP == B200SHM_MAX) asm("max.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+    else asm("min.f64 %0, %1, %2;" : "=d"(r) : "d"(a), "d"(b));
+  } else {
+    r = apply<OP>(a, b);
+  }
+  return r;
+}
+template <int OP, class T>
+__device__ __forceinline__ bool is_zero_of(T v, bool watched) {
+  const bool neg = (OP == B200SHM_MAX) == watched; /* MAX watches for -0, yields +0 */
+  if constexpr (std::is_same<T, float>::value)
+    return __float_as_uint(v) == (neg ? 0x80000000u : 0u);
+  else
+    return (unsigned long long)__double_as_longlong(v) == (neg ? 0x8000000000000000ull : 0ull);
+}
+template <int OP, class T, int V>
+__device__ __forceinline__ Pack<T, V> mm_combine(const Pack<T, V> &a, const Pack<T, V> &b) {
+  Pack<T, V> r;
+#pragma unroll
+  for (int i = 0; i < V; i++) r.x[i] = mm_pick<OP>(a.x[i], b.x[i]);
+  return r;
+}
+template <int OP, class T, int V>
+__device__ __forceinline__ unsigned mm_flags(const Pack<T, V> &v) {
+  if constexpr (std::is_same<T, f80>::value) return pack_class(v);
+  else {
+    unsigned c = 0;
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+      if (is_zero_of<OP>(v.x[i], true)) c |= 1u << i;
+      if constexpr (std::is_same<T, double>::value)
+        if (v.x[i] != v.x[i]) c |= 256u << i;
+    }
+    return c;
+  }
+}
+/* r: the column's combined value, c: its flags */
+template <int OP, class T, int V>
+__device__ __forceinline__ bool mm_ambiguous(const Pack<T, V> &r, unsigned c) {
+  if constexpr (std::is_same<T, f80>::value) return pack_ambiguous(c);
+  else {
+    bool amb = c >= 256u;
+#pragma unroll
+    for (int i = 0; i < V; i++) {
+      amb |= (c >> i & 1u) && is_zero_of<OP>(r.x[i], false);
+      if constexpr (std::is_same<T, float>::value) amb |= r.x[i] != r.x[i];
+    }
+    return amb;
+  }
+}
 
 }  // namespace
 
@@ -286,8 +405,10 @@ struct RArgs {
   char *dst;        /* member 0's dest at element 0            */
   uint64_t sstep;   /* bytes from member i to member i+1 (src) */
   uint64_t dstep;   /* same for dest (equal; kept separate)    */
-  uint64_t e_begin; /* first element of this launch            */
-  uint64_t nvec;    /* packs in this launch                    */
+  uint64_t nvec;    /* packs (or single elements) of the rows' body */
+  unsigned head;    /* elements before the first pack          */
+  unsigned nedge;   /* elements before and after the packs     */
+  int lgG;          /* log2 of the lanes per column            */
   uint64_t N;       /* elements of this view                   */
   uint64_t g_off;   /* the view's element 0 in the whole reduction */
   uint64_t g_n;     /* elements of the whole reduction         */
@@ -300,18 +421,17 @@ struct RArgs {
 
 /* The launch sequence of one validated reduction on stream s, one function
  * per element-type family, each in its own translation unit
- * (reduce_<family>.cu) so the families' kernels compile in parallel.
- * `aligned`: every row starts on a 16-byte boundary. */
-int reduce_dispatch_int(int op, int dtype, const RArgs &a, bool aligned, cudaStream_t s);
-int reduce_dispatch_f32(int op, const RArgs &a, bool aligned, cudaStream_t s);
-int reduce_dispatch_f64(int op, const RArgs &a, bool aligned, cudaStream_t s);
+ * (reduce_<family>.cu) so the families' kernels compile in parallel. */
+int reduce_dispatch_int(int op, int dtype, const RArgs &a, cudaStream_t s);
+int reduce_dispatch_f32(int op, const RArgs &a, cudaStream_t s);
+int reduce_dispatch_f64(int op, const RArgs &a, cudaStream_t s);
 /* long double: one function (and translation unit) per op */
-int reduce_dispatch_f80_min(const RArgs &a, bool aligned, cudaStream_t s);
-int reduce_dispatch_f80_max(const RArgs &a, bool aligned, cudaStream_t s);
-int reduce_dispatch_f80_sum(const RArgs &a, bool aligned, cudaStream_t s);
-int reduce_dispatch_f80_prod(const RArgs &a, bool aligned, cudaStream_t s);
-int reduce_dispatch_c32(int op, const RArgs &a, bool aligned, cudaStream_t s);
-int reduce_dispatch_c64(int op, const RArgs &a, bool aligned, cudaStream_t s);
+int reduce_dispatch_f80_min(const RArgs &a, cudaStream_t s);
+int reduce_dispatch_f80_max(const RArgs &a, cudaStream_t s);
+int reduce_dispatch_f80_sum(const RArgs &a, cudaStream_t s);
+int reduce_dispatch_f80_prod(const RArgs &a, cudaStream_t s);
+int reduce_dispatch_c32(int op, const RArgs &a, cudaStream_t s);
+int reduce_dispatch_c64(int op, const RArgs &a, cudaStream_t s);
 
 namespace {
 
@@ -404,17 +524,136 @@ constexpr int fix_max_members() {
   return sizeof(T) > 8 ? kFixMaxMembersF80 : kFixMaxMembers;
 }
 
+/* shuffles of packs of any size, through 32-bit words */
+template <class T, int V, class F>
+__device__ __forceinline__ Pack<T, V> shfl_words(const Pack<T, V> &v, F shfl) {
+  constexpr int W = ((int)sizeof(v.x) + 3) / 4;
+  uint32_t w[W] = {};
+  memcpy(w, &v, sizeof(v.x));
+#pragma unroll
+  for (int i = 0; i < W; i++) w[i] = shfl(w[i]);
+  Pack<T, V> r;
+  memcpy(&r, w, sizeof(v.x));
+  return r;
+}
+template <class T, int V>
+__device__ __forceinline__ Pack<T, V> shfl_pack(const Pack<T, V> &v, int lane) {
+  return shfl_words(v, [lane](uint32_t x) { return __shfl_sync(0xffffffffu, x, lane); });
+}
+template <class T, int V>
+__device__ __forceinline__ Pack<T, V> shfl_xor_any(const Pack<T, V> &v, int m) {
+  return shfl_words(v, [m](uint32_t x) { return __shfl_xor_sync(0xffffffffu, x, m); });
+}
+
 template <class T, int V>
 __device__ __forceinline__ Pack<T, V> shfl_xor_pack(const Pack<T, V> &v, int m) {
-  static_assert(sizeof(Pack<T, V>) % 4 == 0, "pack of 32-bit words");
-  constexpr int W = (int)(sizeof(Pack<T, V>) / 4);
-  uint32_t w[W];
-  memcpy(w, &v, sizeof(w));
+  return shfl_xor_any(v, m);
+}
+
+
+/* The exact replay inside a warp, for teams whose butterfly has at most
+ * kExactLeaves leaves: V elements from e0 at a time, every lane holding the
+ * inputs of up to 4 members (nodes lane + 32 k) in registers, the
+ * algorithm's own exchange rounds done with shuffles.  All 32 lanes enter;
+ * every input is loaded before any dest is stored, so sources may be dests.
+ * Against a list of deferred elements and a second launch that replays
+ * them, a reduction with none saves that launch. */
+constexpr int kExactLeaves = 64;
+template <class T, int OP, int V>
+__device__ __noinline__ void exact_columns(const RArgs &a, uint64_t e0) {
+  constexpr int K = 2 * kExactLeaves / 32; /* members per lane, at most */
+  typedef Pack<T, V> PK;
+  const int lane = threadIdx.x & 31, P = a.P;
+  const bool bfly = a.algo != B200SHM_LINEAR && a.algo != B200SHM_BINOMIAL;
+  const bool rab = a.algo == B200SHM_RABENSEIFNER || a.algo == B200SHM_RABENSEIFNER2;
+  const int nodes = bfly ? a.p2s : P;
+  const char *src = a.src + e0 * sizeof(T);
+  char *dst = a.dst + e0 * sizeof(T);
+  auto load = [&](int j) { return ld_any<T, V>(src + (uint64_t)j * a.sstep); };
+  auto store = [&](int j, const PK &v) { st_any<T, V>(dst + (uint64_t)j * a.dstep, v); };
+  PK v[K];
+  unsigned cls = 0;
 #pragma unroll
-  for (int i = 0; i < W; i++) w[i] = __shfl_xor_sync(0xffffffffu, w[i], m);
-  Pack<T, V> r;
-  memcpy(&r, w, sizeof(w));
-  return r;
+  for (int k = 0; k < K; k++) {
+    const int q = lane + 32 * k;
+    if (q < nodes) {
+      const int m = bfly ? p2s_member(q, P, a.p2s) : q;
+      v[k] = load(m);
+      cls |= pack_class(v[k]);
+      if (bfly && p2s_extra(q, P, a.p2s)) {
+        const PK x = load(m + 1);
+        cls |= pack_class(x);
+#pragma unroll
+        for (int i = 0; i < V; i++) {
+          /* rec_dbl: op(extra, own) (reduce.c:241); Rabenseifner: that on the
+           * lower half of the vector (397), op(own, extra) on the upper (375) */
+          const bool own_first = rab && a.g_off + e0 + i >= a.g_n / 2;
+          v[k].x[i] = own_first ? apply<OP>(v[k].x[i], x.x[i]) : apply<OP>(x.x[i], v[k].x[i]);
+        }
+      }
+    }
+  }
+  /* the value of node q (the same q in every lane) */
+  auto node = [&](int q, int i) {
+    Pack<T, 1> s;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (k == q >> 5) s.x[0] = v[k].x[i];
+    return shfl_pack(s, q & 31).x[0];
+  };
+  /* a column swept without need may hold its result already */
+  if (!pack_ambiguous(__reduce_or_sync(0xffffffffu, cls))) return; /* all inputs are read */
+  PK r;
+  if (a.algo == B200SHM_LINEAR) { /* a left fold over the members */
+#pragma unroll
+    for (int i = 0; i < V; i++) r.x[i] = node(0, i);
+#pragma unroll 1
+    for (int j = 1; j < P; j++) {
+#pragma unroll
+      for (int i = 0; i < V; i++) r.x[i] = apply<OP>(r.x[i], node(j, i));
+    }
+  } else {
+#pragma unroll 1
+    for (int m = 1; m < nodes; m <<= 1) {
+      PK o[K];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        if (m < 32) {
+          o[k] = shfl_xor_any(v[k], m);
+        } else {
+          o[k] = v[k];
+#pragma unroll
+          for (int h = 1; h < K; h <<= 1)
+            if (m == 32 * h) o[k] = v[k ^ h];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const int q = lane + 32 * k;
+        /* butterfly: member q keeps op(own, partner's) (reduce.c:268, 448);
+         * binomial: the lower member of a pair op(upper block, lower block)
+         * where the upper exists (reduce.c:137-154) */
+        if (bfly) v[k] = papply<OP>(v[k], o[k]);
+        else if ((q & (2 * m - 1)) == 0 && q + m < P) v[k] = papply<OP>(o[k], v[k]);
+      }
+    }
+    if (a.algo == B200SHM_REC_DBL) { /* every p2s member (and its extra) its own value */
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const int q = lane + 32 * k;
+        if (q < nodes) {
+          const int m = p2s_member(q, P, a.p2s);
+          store(m, v[k]);
+          if (p2s_extra(q, P, a.p2s)) store(m + 1, v[k]);
+        }
+      }
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < V; i++) /* the owner of the element's block, or the root */
+      r.x[i] = node(rab ? rev_bits(rab_block(a.g_off + e0 + i, a.g_n, a.p2s), a.logp2s) : 0, i);
+  }
+  for (int j = lane; j < P; j += 32) store(j, r);
 }
 
 }  // namespace

@@ -7,12 +7,12 @@
 
 namespace b200 {
 
-int reduce_dispatch_f64(int op, const RArgs &a, bool aligned, cudaStream_t s) {
+int reduce_dispatch_f64(int op, const RArgs &a, cudaStream_t s) {
   switch (op) {
-  case B200SHM_MIN: return run_float<double, B200SHM_MIN>(a, aligned, s);
-  case B200SHM_MAX: return run_float<double, B200SHM_MAX>(a, aligned, s);
-  case B200SHM_SUM: return run_float<double, B200SHM_SUM>(a, aligned, s);
-  default: return run_float<double, B200SHM_PROD>(a, aligned, s);
+  case B200SHM_MIN: return run_float<double, B200SHM_MIN>(a, s);
+  case B200SHM_MAX: return run_float<double, B200SHM_MAX>(a, s);
+  case B200SHM_SUM: return run_float<double, B200SHM_SUM>(a, s);
+  default: return run_float<double, B200SHM_PROD>(a, s);
   }
 }
 

@@ -9,8 +9,8 @@
 
 namespace b200 {
 
-int reduce_dispatch_f80_max(const RArgs &a, bool aligned, cudaStream_t s) {
-  return run_float<f80, B200SHM_MAX>(a, aligned, s);
+int reduce_dispatch_f80_max(const RArgs &a, cudaStream_t s) {
+  return run_float<f80, B200SHM_MAX>(a, s);
 }
 
 }  // namespace b200

@@ -9,8 +9,8 @@
 
 namespace b200 {
 
-int reduce_dispatch_f80_prod(const RArgs &a, bool aligned, cudaStream_t s) {
-  return run_float<f80, B200SHM_PROD>(a, aligned, s);
+int reduce_dispatch_f80_prod(const RArgs &a, cudaStream_t s) {
+  return run_float<f80, B200SHM_PROD>(a, s);
 }
 
 }  // namespace b200

@@ -27,12 +27,29 @@
  *    after folding the extra members (reduce.c:206-272, 338-454) -- the
  *    same tree for all three;
  *  - float MIN/MAX written a<b?a:b (reduce.c:731-732) is order dependent
- *    only when the operands include a NaN or both +0 and -0; elements with
- *    such operands take an exact per-member path that replays the
- *    algorithm's operand order (rec_dbl then gives different members
- *    different bits, exactly as the reference does).
- * Trees are evaluated as a binary counter over the leaves, with one
- * register slot per tree level, so leaves stream in member order.
+ *    only when the operands include a NaN or both +0 and -0; columns with
+ *    such operands are replayed in the algorithm's operand order, by their
+ *    warp in the same launch (exact_columns; teams whose butterfly has more
+ *    than 64 leaves: k_minmax_fix).  rec_dbl then gives different members
+ *    different bits, exactly as the reference does.
+ * Trees over more than 32 leaves in a lane are evaluated as a binary counter
+ * over subtrees of 8, with one register slot per level, so leaves stream in
+ * member order.
+ *
+ * What the kernel is bound by, and measured (GB/s of 2*P*N*sizeof(T); us in
+ * a graph of back-to-back calls), against one launch for the packs with one
+ * or two lanes a column, a second for the last elements, single elements
+ * throughout where rows leave the 16-byte grid, and a replay launch after
+ * every float MIN/MAX:
+ *   64 members x 2^20, f32 SUM / f64 MAX / i64 XOR in a row: HBM, 6.15 TB/s
+ *   before and after (437.0 and 435.4 us);
+ *   100 members x 50001 doubles, one element off the grid, rabenseifner
+ *   order: 0.62 -> 4.1 TB/s (129 -> 19.2 us), HBM and the loads in flight of
+ *   a lane's 16 leaves and their extras;
+ *   64 members x 4096: f32 SUM 5.6 -> 2.6 us, f64 MAX 10.9 -> 3.8 us, latency
+ *   of the launch and of one or two rounds of loads;
+ *   2 members x 65536 f64 MAX 4.5 -> 2.5 us; 64 members x 2^20 int16 SUM off
+ *   the grid 144 -> 52 us; 100 x 2^16 complex double SUM 78 -> 52 us.
  * No fused multiply-add is ever formed: float ops use the _rn intrinsics.
  */
 #pragma once
@@ -40,6 +57,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
 #include <mutex>
 #include <type_traits>
 #include <unordered_map>
@@ -51,8 +69,10 @@
 namespace b200 {
 namespace {
 
-/* Second pass over the elements the streaming kernel deferred (it left
- * their dests untouched, so in-place sources are still intact): one CTA
+/* Teams of more than 2 * kExactLeaves - 1 members only (smaller ones replay
+ * such elements inside the streaming kernel, exact_columns): second pass
+ * over the elements the streaming kernel deferred (it left their dests
+ * untouched, so in-place sources are still intact): one CTA
  * per element stages the P inputs in shared memory, then replays the
  * algorithm's operand order from there.  Launched as a programmatic
  * dependent of the streaming kernel: its CTAs may become resident during
@@ -119,314 +139,380 @@ __device__ __forceinline__ void allow_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-/* ---- the streaming kernels -------------------------------------------- */
-template <class T, int OP, int ORDER, int V, int U, bool MINMAX_CHECK, int LV>
-__global__ void __launch_bounds__(256) k_reduce(const RArgs a) {
-  typedef Pack<T, V> PK;
-  if constexpr (MINMAX_CHECK) allow_dependents();
-  /* grid-stride: all CTAs sweep one contiguous front of every member's
-   * slice together, which keeps DRAM row locality (contiguous per-CTA
-   * ranges measured ~20% slower) */
-  const uint64_t gstride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < a.nvec; v += gstride) {
-    const uint64_t e0 = a.e_begin + v * V;
-    const char *src = a.src + e0 * sizeof(T);
-    PK r;
-    unsigned cls[V];
-    if constexpr (ORDER == ORD_CHAIN) {
-      r = ld_pack<T, V>(src);
-      if constexpr (MINMAX_CHECK) {
-#pragma unroll
-        for (int i = 0; i < V; i++) cls[i] = fclass(r.x[i]);
-      }
-      for (int j = 1; j < a.P; j += U) {
-        PK x[U];
-#pragma unroll
-        for (int u = 0; u < U; u++)
-          if (j + u < a.P) x[u] = ld_pack<T, V>(src + (uint64_t)(j + u) * a.sstep);
-#pragma unroll
-        for (int u = 0; u < U; u++)
-          if (j + u < a.P) {
-            r = papply<OP>(r, x[u]);
-            if constexpr (MINMAX_CHECK) {
-#pragma unroll
-              for (int i = 0; i < V; i++) cls[i] |= fclass(x[u].x[i]);
-            }
-          }
-      }
+/* ---- the streaming kernel ----------------------------------------------
+ * A column is V consecutive elements of every member (one 16-byte pack), or
+ * one element where packs do not apply.  G lanes (a power of two) share a
+ * column.  Lane g owns a contiguous share of the leaves -- for the
+ * butterfly and for binomial trees over a power-of-two team that share is a
+ * complete subtree -- and reduces it from loads it keeps up to 8 deep; the G
+ * partial results are then combined across lanes with __shfl_xor over masks
+ * 1, 2, ..., G/2, which is exactly the butterfly's remaining levels (mask m
+ * pairs group g with g^m, lower group first: reduce.c:250-272).  Every lane
+ * then stores the result to its own share of the members.
+ *
+ * How a column is accessed (MODE):
+ *   kPacks    16-byte accesses: every row has the same offset from the
+ *             16-byte grid, so the columns begin at the grid's first point
+ *             in the rows and the elements before it and after the last
+ *             whole pack (at most 2(V-1)) are columns of one element, in
+ *             the same launch;
+ *   kElements one element each, at its own alignment: rows of different
+ *             offsets (dest and source shifted against each other, member
+ *             strides off the grid);
+ *   kBytes    elements at any byte offset. */
+enum { kPacks = 0, kElements = 1, kBytes = 2 };
+
+template <class T, int V, int MODE>
+__device__ __forceinline__ Pack<T, V> ld_col(const char *p) {
+  if constexpr (MODE == kPacks && sizeof(T) == 16) {
+    uint32_t w[4];
+    asm(B200_LD_OP ".v4.u32 {%0,%1,%2,%3}, [%4];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+        : "l"(p));
+    Pack<T, V> r;
+    memcpy(&r, w, 16);
+    return r;
+  } else if constexpr (MODE == kElements) {
+    static_assert(V == 1 && sizeof(T) <= 8, "one element at its own alignment");
+    Pack<T, V> r;
+    if constexpr (sizeof(T) == 8) {
+      unsigned long long u;
+      asm(B200_LD_OP ".u64 %0, [%1];" : "=l"(u) : "l"(p));
+      memcpy(&r, &u, 8);
+    } else if constexpr (sizeof(T) == 4) {
+      unsigned u;
+      asm(B200_LD_OP ".u32 %0, [%1];" : "=r"(u) : "l"(p));
+      memcpy(&r, &u, 4);
+    } else if constexpr (sizeof(T) == 2) {
+      unsigned short u;
+      asm(B200_LD_OP ".u16 %0, [%1];" : "=h"(u) : "l"(p));
+      memcpy(&r, &u, 2);
     } else {
-      PK stk[LV]; /* LV levels hold trees of up to 2^LV - 1 leaves */
-      const int nleaves = ORDER == ORD_BUTTERFLY ? a.p2s : a.P;
-      /* comb(lower block, upper block) in the algorithm's operand order */
-      auto comb = [](const PK &lo, const PK &hi) {
-        return ORDER == ORD_BUTTERFLY ? papply<OP>(lo, hi) : papply<OP>(hi, lo);
-      };
-      /* binary counter: pushing block number q at level `base` closes
-       * t = trailing_ones(q) blocks and parks the result at level base+t
-       * (all register indices static) */
-      auto push = [&](PK y, int q, int base) {
-        const int t = base + __ffs(~q) - 1;
-#pragma unroll
-        for (int L = 0; L < LV - 1; L++)
-          if (L >= base && L < t) y = comb(stk[L], y);
-#pragma unroll
-        for (int L = 0; L < LV; L++)
-          if (L == t) stk[L] = y;
-      };
-      /* p2s member q is member ceil(q*P/p2s) (p2s is a power of two, so the
-       * division is a shift); it has an extra member folded into it exactly
-       * when the next p2s member is two members further on */
-      auto member_of = [&](int q) -> int {
-        return ORDER == ORD_BUTTERFLY
-                   ? (int)(((long long)q * a.P + a.p2s - 1) >> a.logp2s)
-                   : q;
-      };
-      auto leaf_addr = [&](int q) { return src + (uint64_t)member_of(q) * a.sstep; };
-      auto fold_extra = [&](PK &x, int q) {
-        /* rec_dbl / Rabenseifner fold the extra member in first as
-         * op(extra, own) (reduce.c:232-241) */
-        if (ORDER == ORD_BUTTERFLY && a.P != a.p2s && member_of(q + 1) - member_of(q) == 2)
-          x = papply<OP>(ld_pack<T, V>(leaf_addr(q) + a.sstep), x);
-      };
-      int q0 = 0;
-      /* full chunks of 8 leaves: 8 loads in flight, a fixed 8-leaf subtree */
-      for (; q0 + 8 <= nleaves; q0 += 8) {
-        PK x[8];
-#pragma unroll
-        for (int u = 0; u < 8; u++) x[u] = ld_pack<T, V>(leaf_addr(q0 + u));
-#pragma unroll
-        for (int u = 0; u < 8; u++) fold_extra(x[u], q0 + u);
-        const PK c = comb(comb(comb(x[0], x[1]), comb(x[2], x[3])),
-                          comb(comb(x[4], x[5]), comb(x[6], x[7])));
-        push(c, q0 >> 3, 3);
-      }
-      /* the last < 8 leaves (trees of < 8 leaves, binomial with P % 8 != 0) */
-#pragma unroll 1
-      for (; q0 < nleaves; q0++) {
-        PK x = ld_pack<T, V>(leaf_addr(q0));
-        fold_extra(x, q0);
-        push(x, q0, 0);
-      }
-      if constexpr (ORDER == ORD_BUTTERFLY) {
-#pragma unroll
-        for (int L = 0; L < LV; L++)
-          if (L == a.logp2s) r = stk[L];
-      } else {
-        bool have = false;
-#pragma unroll
-        for (int L = 0; L < LV; L++)
-          if (a.P & (1 << L)) {
-            r = have ? papply<OP>(r, stk[L]) : stk[L];
-            have = true;
-          }
-      }
+      unsigned u;
+      asm(B200_LD_OP ".u8 %0, [%1];" : "=r"(u) : "l"(p));
+      const unsigned char c = (unsigned char)u;
+      memcpy(&r, &c, 1);
     }
-    if constexpr (MINMAX_CHECK) {
-      bool amb = false;
-#pragma unroll
-      for (int i = 0; i < V; i++) amb |= ambiguous(cls[i]);
-      if (amb) {
-        /* defer the whole pack; its dests stay untouched until k_minmax_fix */
-        const unsigned long long slot = atomicAdd(a.fix_count, (unsigned long long)V);
-        for (int i = 0; i < V; i++) {
-          if (slot + i < a.fix_cap) a.fix_list[slot + i] = e0 + i;
-          else atomicOr(a.status, (int)B200SHM_STATUS_FIX_OVERFLOW);
-        }
-        continue;
-      }
+    return r;
+  } else {
+    return ld_pack<T, V>(p);
+  }
+}
+template <class T, int V, int MODE>
+__device__ __forceinline__ void st_col(char *p, const Pack<T, V> &v) {
+  if constexpr (MODE == kPacks && sizeof(T) == 16) {
+    uint32_t w[4];
+    memcpy(w, &v, 16);
+    asm volatile(B200_ST_OP ".v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(w[0]), "r"(w[1]),
+                 "r"(w[2]), "r"(w[3])
+                 : "memory");
+  } else if constexpr (MODE == kElements) {
+    if constexpr (sizeof(T) == 8) {
+      unsigned long long u;
+      memcpy(&u, &v, 8);
+      asm volatile(B200_ST_OP ".u64 [%0], %1;" ::"l"(p), "l"(u) : "memory");
+    } else if constexpr (sizeof(T) == 4) {
+      unsigned u;
+      memcpy(&u, &v, 4);
+      asm volatile(B200_ST_OP ".u32 [%0], %1;" ::"l"(p), "r"(u) : "memory");
+    } else if constexpr (sizeof(T) == 2) {
+      unsigned short u;
+      memcpy(&u, &v, 2);
+      asm volatile(B200_ST_OP ".u16 [%0], %1;" ::"l"(p), "h"(u) : "memory");
+    } else {
+      unsigned char c;
+      memcpy(&c, &v, 1);
+      asm volatile(B200_ST_OP ".u8 [%0], %1;" ::"l"(p), "r"((unsigned)c) : "memory");
     }
-    char *dst = a.dst + e0 * sizeof(T);
-    for (int j = 0; j < a.P; j++) st_pack<T, V>(dst + (uint64_t)j * a.dstep, r);
+  } else {
+    st_pack<T, V>(p, v);
   }
 }
 
-/* Launch the packed body over [0, N - N%V) and a scalar tail, or scalar
- * throughout when the buffers are not 16-byte aligned. */
-/* ---- warp-cooperative variant ----------------------------------------
- * G lanes (a power of two) share one 16-byte column.  Lane group g owns a
- * contiguous share of the leaves -- for the butterfly and for binomial
- * trees over a power-of-two team that share is a complete subtree -- and
- * reduces it from loads it keeps 8 deep; the G partial results are then
- * combined across lanes with __shfl_xor over masks 1, 2, ..., G/2, which
- * is exactly the butterfly's remaining levels (mask m pairs group g with
- * g^m, lower group first: reduce.c:250-272).  Every lane then stores the
- * result to its own share of the members.  Registers per lane no longer
- * grow with the tree depth, and a pack's 2*P memory operations are spread
- * over G lanes. */
+/* A lane's place: its column group, its leaves [l0, l1) and the members
+ * [m0, m1) it stores to. */
+struct Lane {
+  int G, g, l0, l1, m0, m1;
+};
 
-/* The MIN/MAX-checking instances take 78 registers (3 CTAs per SM), the
- * others 48 (5).  Holding the MIN/MAX ones to 64 (4 CTAs per SM, no spills)
- * measured slower on the 64-PE headline (f64 MAX 5908-5912 against
- * 5938-5950 GB/s), so they are left unbounded. */
-template <class T, int OP, int ORDER, int V, int G, bool MM, int LVL, bool POW2>
-__global__ void __launch_bounds__(256) k_reduce_coop(const RArgs a) {
+/* One column group's work on the column whose first element is e0 (live:
+ * the column exists; the whole warp enters, for the shuffles).  C: leaves a
+ * lane of a tree holds -- 2, 4, 8: all loaded at once; 16, 32: chunks of 8;
+ * 0: any number of chunks of 8, a binary counter over them; kRagged<L>:
+ * fewer than 2^L leaves, not a power of two (a binomial tree in one lane):
+ * chunks of 8, then the last leaves one by one.
+ * True for a MIN/MAX column whose bits depend on operand order: its dests
+ * are left for the exact replay. */
+template <int LEVELS>
+constexpr int kRagged = -LEVELS;
+template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2, int MODE>
+__device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, uint64_t e0,
+                                              bool live) {
   typedef Pack<T, V> PK;
-  if constexpr (MM) allow_dependents();
-  constexpr int COLS = 32 / G; /* packs per warp per iteration */
-  const int lane = threadIdx.x & 31;
-  const int g = lane & (G - 1), c = lane / G;
-  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  const int P = a.P;
-  const int nleaves = ORDER == ORD_BUTTERFLY ? a.p2s : P;
-  /* this lane's leaves [l0, l1) */
-  const int l0 = (int)((long long)g * nleaves / G), l1 = (int)((long long)(g + 1) * nleaves / G);
-  /* members this lane stores to: [m0, m1) */
-  int m0, m1;
-  if (ORDER == ORD_BUTTERFLY) {
-    m0 = (int)(((long long)l0 * P + a.p2s - 1) >> a.logp2s);
-    m1 = (int)(((long long)l1 * P + a.p2s - 1) >> a.logp2s);
-  } else {
-    m0 = l0;
-    m1 = l1;
-  }
+  const int P = a.P, l0 = ln.l0, l1 = ln.l1;
   auto member_of = [&](int q) -> int {
-    return ORDER == ORD_BUTTERFLY ? (int)(((long long)q * P + a.p2s - 1) >> a.logp2s) : q;
+    /* trees have at most 2^13 members: no overflow */
+    return ORDER == ORD_BUTTERFLY ? (q * P + a.p2s - 1) >> a.logp2s : q;
   };
   auto comb = [](const PK &lo, const PK &hi) {
-    if constexpr (ORDER == ORD_BINOMIAL) return papply<OP>(hi, lo);
+    if constexpr (MM) return mm_combine<OP>(lo, hi);
+    else if constexpr (ORDER == ORD_BINOMIAL) return papply<OP>(hi, lo);
     else return papply<OP>(lo, hi);
   };
-  for (uint64_t base = warp * COLS; base < a.nvec; base += nwarps * COLS) {
-    const uint64_t v = base + c;
-    const bool live = v < a.nvec; /* uniform per column group */
-    const uint64_t e0 = a.e_begin + (live ? v : 0) * V;
-    const char *src = a.src + e0 * sizeof(T);
-    PK r;
-    unsigned cls[V];
+  const char *src = a.src + e0 * sizeof(T);
+  PK r;
+  unsigned cls = 0;
+  if (live) {
+    if constexpr (ORDER == ORD_CHAIN) {
+      const char *p = src + (uint64_t)l0 * a.sstep;
+      r = ld_col<T, V, MODE>(p);
+      int j = l0 + 1;
+      do { /* once at least: a MIN/MAX lane looks at its first operand below the loads */
+        PK x[8];
+        const uint64_t step = opaque(a.sstep);
 #pragma unroll
-    for (int i = 0; i < V; i++) cls[i] = 0;
-    if (live) {
-      if constexpr (ORDER == ORD_CHAIN) {
-        r = ld_pack<T, V>(src + (uint64_t)l0 * a.sstep);
-        if constexpr (MM) {
+        for (int u = 0; u < 8; u++)
+          if (j + u < l1) x[u] = ld_col<T, V, MODE>(p + (uint64_t)(u + 1) * step);
+        p += 8 * step;
+        if constexpr (MM)
+          if (j == l0 + 1) cls = mm_flags<OP>(r);
 #pragma unroll
-          for (int i = 0; i < V; i++) cls[i] = fclass(r.x[i]);
-        }
-        for (int j = l0 + 1; j < l1; j += 8) {
-          PK x[8];
+        for (int u = 0; u < 8; u++)
+          if (j + u < l1) {
+            r = comb(r, x[u]);
+            if constexpr (MM) cls |= mm_flags<OP>(x[u]);
+          }
+        j += 8;
+      } while (j < l1);
+    } else {
+      /* K leaves from q0 as a complete subtree, all loads before any use;
+       * extra members folded in first as op(extra, own) (reduce.c:232-241) */
+      auto chunk = [&](int q0, auto k_c) {
+        constexpr int K = decltype(k_c)::value;
+        PK x[K];
+        if constexpr (POW2 || ORDER == ORD_BINOMIAL) { /* member == leaf */
+          const uint64_t step = a.sstep;
+          const char *p = src + (uint64_t)q0 * step;
 #pragma unroll
-          for (int u = 0; u < 8; u++)
-            if (j + u < l1) x[u] = ld_pack<T, V>(src + (uint64_t)(j + u) * a.sstep);
+          for (int u = 0; u < K; u++) x[u] = ld_col<T, V, MODE>(p + (uint64_t)u * step);
+        } else {
 #pragma unroll
-          for (int u = 0; u < 8; u++)
-            if (j + u < l1) {
-              r = papply<OP>(r, x[u]);
-              if constexpr (MM) {
+          for (int h = 0; h < K; h += 4) { /* up to 4 leaves and their extras in flight */
+            constexpr int E = K < 4 ? K : 4;
+            const uint64_t step = opaque(a.sstep);
+            const char *p = src + (uint64_t)member_of(q0 + h) * step;
+            PK e[E];
+            bool ex[E];
 #pragma unroll
-                for (int i = 0; i < V; i++) cls[i] |= fclass(x[u].x[i]);
+            for (int u = 0; u < E; u++, p += step) {
+              x[h + u] = ld_col<T, V, MODE>(p);
+              ex[u] = member_of(q0 + h + u + 1) - member_of(q0 + h + u) == 2;
+              if (ex[u]) {
+                p += step;
+                e[u] = ld_col<T, V, MODE>(p);
               }
             }
+#pragma unroll
+            for (int u = 0; u < E; u++)
+              if (ex[u]) x[h + u] = papply<OP>(e[u], x[h + u]);
+          }
+        }
+#pragma unroll
+        for (int w = K; w > 1; w >>= 1) {
+#pragma unroll
+          for (int i = 0; i < w / 2; i++) x[i] = comb(x[2 * i], x[2 * i + 1]);
+        }
+        return x[0];
+      };
+      typedef std::integral_constant<int, 8> k8;
+      if constexpr (C >= 2 && C <= 8) {
+        r = chunk(l0, std::integral_constant<int, C>{});
+      } else if constexpr (C == 16) {
+        /* two chunks, one at a time (keeps 8 loads in flight, not 16) */
+#pragma unroll 1
+        for (int c2 = 0; c2 < 2; c2++) {
+          const PK y = chunk(l0 + 8 * c2, k8{});
+          r = c2 ? comb(r, y) : y;
+        }
+      } else if constexpr (C == 32) {
+        /* four chunks, one at a time: ((c0 c1)(c2 c3)) with two slots */
+        PK h, s2;
+#pragma unroll 1
+        for (int c4 = 0; c4 < 4; c4++) {
+          PK y = chunk(l0 + 8 * c4, k8{});
+          if (c4 & 1) {
+            y = comb(h, y);
+            if (c4 == 1) s2 = y;
+            else r = comb(s2, y);
+          } else {
+            h = y;
+          }
         }
       } else {
-        /* complete subtree of l1-l0 (a power of two) leaves: chunks of 8
-         * as fixed subtrees; LVL == 1: one chunk, LVL == 2: two chunks, LVL == 4: four,
-         * else a counter over the chunks (LVL levels hold 2^(LVL-1)) */
+        constexpr bool kRest = C < 0;
+        constexpr int LV = kRest ? -C : kMaxLevels - 3; /* levels of 2^k leaves (chunks) */
+        PK stk[LV];
         const int n = l1 - l0;
-        auto chunk = [&](int q0) {
-          PK x[8];
-          if constexpr (POW2) { /* member == leaf */
-            const char *p = src + (uint64_t)q0 * a.sstep;
+        int c = 0; /* subtrees of the lowest level pushed so far */
+        auto push = [&](PK y, int lv) {
+          const int t = lv + __ffs(~(c >> lv)) - 1;
 #pragma unroll
-            for (int u = 0; u < 8; u++) x[u] = ld_pack<T, V>(p + (uint64_t)u * a.sstep);
-          } else {
+          for (int L = 0; L < LV - 1; L++)
+            if (L >= lv && L < t) y = comb(stk[L], y);
 #pragma unroll
-            for (int u = 0; u < 8; u++) x[u] = ld_pack<T, V>(src + (uint64_t)member_of(q0 + u) * a.sstep);
-#pragma unroll
-            for (int u = 0; u < 8; u++) /* op(extra, own), reduce.c:232-241 */
-              if (member_of(q0 + u + 1) - member_of(q0 + u) == 2)
-                x[u] = papply<OP>(ld_pack<T, V>(src + (uint64_t)(member_of(q0 + u) + 1) * a.sstep), x[u]);
-          }
-          return comb(comb(comb(x[0], x[1]), comb(x[2], x[3])), comb(comb(x[4], x[5]), comb(x[6], x[7])));
+          for (int L = 0; L < LV; L++)
+            if (L == t) stk[L] = y;
+          c += 1 << lv;
         };
-        if constexpr (LVL == 1) {
-          r = chunk(l0);
-        } else if constexpr (LVL == 2) {
-          /* two chunks, one at a time (keeps 8 loads in flight, not 16) */
-#pragma unroll 1
-          for (int c2 = 0; c2 < 2; c2++) {
-            const PK y = chunk(l0 + 8 * c2);
-            r = c2 ? comb(r, y) : y;
-          }
-        } else if constexpr (LVL == 4) {
-          /* four chunks, one at a time: ((c0 c1)(c2 c3)) with two slots */
-          PK h, s2;
-#pragma unroll 1
-          for (int c4 = 0; c4 < 4; c4++) {
-            PK y = chunk(l0 + 8 * c4);
-            if (c4 & 1) {
-              y = comb(h, y);
-              if (c4 == 1) s2 = y;
-              else r = comb(s2, y);
-            } else {
-              h = y;
+        int q = 0;
+        if constexpr (LV > 3)
+          for (; q + 8 <= n; q += 8) push(chunk(l0 + q, k8{}), kRest ? 3 : 0);
+        if constexpr (kRest) {
+          PK x[7];
+#pragma unroll
+          for (int u = 0; u < 7; u++)
+            if (q + u < n) x[u] = ld_col<T, V, MODE>(src + (uint64_t)(q + u) * a.sstep);
+#pragma unroll
+          for (int u = 0; u < 7; u++)
+            if (q + u < n) push(x[u], 0);
+          bool have = false;
+#pragma unroll
+          for (int L = 0; L < LV; L++)
+            if (n & (1 << L)) {
+              r = have ? papply<OP>(r, stk[L]) : stk[L];
+              have = true;
             }
-          }
         } else {
-          PK stk[LVL];
-          for (int q0 = 0; q0 < n; q0 += 8) {
-            PK y = chunk(l0 + q0);
-            const int sidx = q0 >> 3, t = __ffs(~sidx) - 1;
-#pragma unroll
-            for (int L = 0; L < LVL - 1; L++)
-              if (L < t) y = comb(stk[L], y);
-#pragma unroll
-            for (int L = 0; L < LVL; L++)
-              if (L == t) stk[L] = y;
-          }
           const int top = __ffs(n >> 3) - 1; /* log2(n/8) */
 #pragma unroll
-          for (int L = 0; L < LVL; L++)
+          for (int L = 0; L < LV; L++)
             if (L == top) r = stk[L];
         }
       }
     }
-    /* butterfly levels across the G lanes of this column */
-#pragma unroll
-    for (int m = 1; m < G; m <<= 1) {
-      const PK o = shfl_xor_pack<T, V>(r, m);
-      r = (g & m) ? comb(o, r) : comb(r, o);
-      if constexpr (MM) {
-#pragma unroll
-        for (int i = 0; i < V; i++) cls[i] |= __shfl_xor_sync(0xffffffffu, cls[i], m);
+  }
+  /* butterfly levels across the G lanes of this column */
+  for (int m = 1; m < ln.G; m <<= 1) {
+    const PK o = shfl_xor_pack<T, V>(r, m);
+    r = (ln.g & m) ? comb(o, r) : comb(r, o);
+    if constexpr (MM) cls |= __shfl_xor_sync(0xffffffffu, cls, m);
+  }
+  if constexpr (MM) {
+    const bool amb = live && mm_ambiguous<OP>(r, cls);
+    if (amb && ln.g == 0 && a.fix_list != nullptr) { /* on the list of deferred elements */
+      const unsigned long long slot = atomicAdd(a.fix_count, (unsigned long long)V);
+      for (int i = 0; i < V; i++) {
+        if (slot + i < a.fix_cap) a.fix_list[slot + i] = e0 + i;
+        else atomicOr(a.status, (int)B200SHM_STATUS_FIX_OVERFLOW);
       }
     }
-    if (!live) continue;
-    if constexpr (MM) {
-      bool amb = false;
-#pragma unroll
-      for (int i = 0; i < V; i++) amb |= ambiguous(cls[i]);
-      if (amb) { /* defer the pack; its dests stay untouched */
-        if (g == 0) {
-          const unsigned long long slot = atomicAdd(a.fix_count, (unsigned long long)V);
-          for (int i = 0; i < V; i++) {
-            if (slot + i < a.fix_cap) a.fix_list[slot + i] = e0 + i;
-            else atomicOr(a.status, (int)B200SHM_STATUS_FIX_OVERFLOW);
-          }
-        }
-        continue;
-      }
+    if (amb) return true;
+  }
+  if (!live) return false;
+  char *dst = a.dst + e0 * sizeof(T) + (uint64_t)ln.m0 * a.dstep;
+  for (int j = ln.m0; j < ln.m1; j++, dst += a.dstep) st_col<T, V, MODE>(dst, r);
+  return false;
+}
+
+/* The columns a warp left in its turns (see k_reduce), replayed exactly.
+ * After the streaming loop and out of line, so that the loop's registers
+ * and code are those of a kernel without it. */
+template <class T, int OP, int V>
+__device__ __noinline__ void exact_sweep(const RArgs &a, unsigned left, int lgG, uint64_t warp,
+                                         uint64_t nwarps, uint64_t nb) {
+  const int lgcols = 5 - lgG;
+  unsigned turn = 1;
+  for (uint64_t t = warp; t < nb; t += nwarps) {
+    unsigned todo = __ballot_sync(0xffffffffu, (left & turn) != 0);
+    for (; todo; todo &= todo - 1) {
+      const uint64_t v = (t << lgcols) + ((__ffs(todo) - 1) >> lgG);
+      if (v < a.nvec) exact_columns<T, OP, V>(a, a.head + v * V);
     }
-    char *dst = a.dst + e0 * sizeof(T);
-    for (int j = m0; j < m1; j++) st_pack<T, V>(dst + (uint64_t)j * a.dstep, r);
+    if (turn != 1u << 31) turn <<= 1;
   }
 }
 
-/* Grid for one register-path launch: at most `occ` CTAs per SM (8 unless
- * B200SHM_REDUCE_CTAS_PER_SM overrides it for tuning sweeps); CTAs
- * grid-stride over the packs. */
-template <class K>
-unsigned reduce_grid(K kernel, int &occ, uint64_t nvec, int threads) {
-  (void)kernel;
-  if (occ < 0) { /* cached per kernel instantiation by the caller */
-    int o = 8; /* oversubscribed grid-stride grid: measured best */
-    const char *env = getenv("B200SHM_REDUCE_CTAS_PER_SM");
-    if (env && atoi(env) > 0) o = atoi(env);
-    occ = o;
+/* The elements before and after the packs, columns of one element, the last
+ * warps first. */
+template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2>
+__device__ __forceinline__ void reduce_edges(const RArgs &a, const Lane &ln, int lgG,
+                                             uint64_t warp, uint64_t nwarps) {
+  const int c = (threadIdx.x & 31) >> lgG, lgcols = 5 - lgG;
+  const unsigned ne = (a.nedge + (1u << lgcols) - 1) >> lgcols;
+  for (uint64_t t = warp; t < ne; t += nwarps) {
+    const unsigned i = (unsigned)(t << lgcols) + c;
+    const bool live = i < a.nedge;
+    const uint64_t e = !live ? 0 : i < a.head ? i : i + a.nvec * V;
+    const bool amb = reduce_column<T, OP, ORDER, 1, MM, C, POW2, kElements>(a, ln, e, live);
+    if constexpr (MM) {
+      if (a.fix_list == nullptr) {
+        unsigned todo = __ballot_sync(0xffffffffu, amb && ln.g == 0);
+        for (; todo; todo &= todo - 1)
+          exact_columns<T, OP, 1>(a, __shfl_sync(0xffffffffu, e, __ffs(todo) - 1));
+      }
+    }
   }
-  const uint64_t need = (nvec + threads - 1) / threads;
-  const uint64_t cap = (uint64_t)grid_sms() * (uint64_t)occ;
-  return (unsigned)(need < cap ? (need ? need : 1) : cap);
+}
+
+/* CTAs per SM an instance is held to, at least: 5 (48 registers) where it
+ * fits without spills (trees, chains of 8-byte elements), 4 with 4-byte
+ * elements or with edges (the code for single elements costs registers, so
+ * rows of whole packs, nedge == 0, have an instance without it), 2 with
+ * smaller elements (unpacked into a register each); 3 for the MIN/MAX ones:
+ * holding those to 64 registers (4 CTAs per SM, no spills) measured slower
+ * on the 64-PE headline (f64 MAX 5908-5912 against 5938-5950 GB/s). */
+template <class T, int ORDER, bool MM, int C, bool POW2, int MODE, bool EDGES>
+constexpr int min_ctas() {
+  if (MODE == kBytes) return 1;
+  if (MM) return 3;
+  if (ORDER == ORD_CHAIN) return sizeof(T) < 4 ? 2 : sizeof(T) == 4 || EDGES ? 4 : 5;
+  return C == 0 || C < -3 ? 2 : !POW2 ? 3 : EDGES ? 4 : 5;
+}
+template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2, int MODE, bool EDGES>
+__global__ void __launch_bounds__(256, min_ctas<T, ORDER, MM, C, POW2, MODE, EDGES>())
+k_reduce(const __grid_constant__ RArgs a) {
+  if constexpr (MM) allow_dependents();
+  const int lane = threadIdx.x & 31, lgG = a.lgG;
+  Lane ln;
+  ln.G = 1 << lgG;
+  ln.g = lane & (ln.G - 1);
+  const int c = lane >> lgG, lgcols = 5 - lgG; /* columns per warp per iteration */
+  const int P = a.P;
+  const int nleaves = ORDER == ORD_BUTTERFLY ? a.p2s : P;
+  ln.l0 = (ln.g * nleaves) >> lgG; /* at most 2^20 members, 16 lanes */
+  ln.l1 = ((ln.g + 1) * nleaves) >> lgG;
+  if (ORDER == ORD_BUTTERFLY) {
+    ln.m0 = (ln.l0 * P + a.p2s - 1) >> a.logp2s;
+    ln.m1 = (ln.l1 * P + a.p2s - 1) >> a.logp2s;
+  } else {
+    ln.m0 = ln.l0;
+    ln.m1 = ln.l1;
+  }
+  /* grid-stride: all CTAs sweep one contiguous front of every member's
+   * slice together, which keeps DRAM row locality (contiguous per-CTA
+   * ranges measured ~20% slower) */
+  const uint64_t warp = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint64_t nwarps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  const uint64_t nb = (a.nvec + (1u << lgcols) - 1) >> lgcols;
+  unsigned left = 0; /* bit i: this lane's column of turn i (the last bit: and of
+                      * the turns after it) is left for the exact replay */
+  unsigned turn = 1;
+  for (uint64_t t = warp; t < nb; t += nwarps) {
+    const uint64_t v = (t << lgcols) + c;
+    const bool live = v < a.nvec;
+    const bool amb = reduce_column<T, OP, ORDER, V, MM, C, POW2, MODE>(
+        a, ln, a.head + (live ? v : 0) * V, live);
+    if constexpr (MM) {
+      if (amb && ln.g == 0) left |= turn;
+      if (turn != 1u << 31) turn <<= 1;
+    }
+  }
+  if constexpr (MM) {
+    if (a.fix_list == nullptr && __any_sync(0xffffffffu, left != 0))
+      exact_sweep<T, OP, V>(a, left, lgG, warp, nwarps, nb);
+  }
+  if constexpr (EDGES)
+    reduce_edges<T, OP, ORDER, V, MM, C, POW2>(a, ln, lgG, nwarps - 1 - warp, nwarps);
 }
 
 /* CTAs of 256 threads of `kernel` that one SM holds at once (cached per
@@ -446,130 +532,136 @@ int resident_ctas(const void *kernel) {
   return n;
 }
 
-/* Grid of the warp-cooperative kernel, in waves of the CTAs one SM holds
- * at once: 8 waves by default (B200SHM_REDUCE_WAVES overrides it, or
+/* Launch over `lanes` threads of work.  Grid: up to 8 waves of the CTAs one
+ * SM holds at once (B200SHM_REDUCE_WAVES overrides it, or
  * B200SHM_REDUCE_CTAS_PER_SM gives a fixed count).  On the 64-PE x 2^20
- * workload one exact wave was slowest (5.27 TB/s over the six
- * reductions): CTAs of a grid-stride loop finish unevenly and leave their
- * SM's slots idle, while the CTAs of later waves backfill them.  4 waves
- * gave 5.73, 6-16 waves 5.78-5.80, one pack per lane 5.76. */
-unsigned coop_grid(const void *kernel, uint64_t lanes) {
+ * workload one exact wave was slowest (5.27 TB/s over the six reductions):
+ * CTAs of a grid-stride loop finish unevenly and leave their SM's slots
+ * idle, while the CTAs of later waves backfill them.  4 waves gave 5.73,
+ * 6-16 waves 5.78-5.80, one pack per lane 5.76.  CTAs of 256 threads, less
+ * where that leaves SMs without one. */
+template <class K>
+void launch_one(K kernel, uint64_t lanes, cudaStream_t s, const RArgs &a) {
   static int per_sm_env = -1, waves = 8;
   if (per_sm_env < 0) {
     const char *e = getenv("B200SHM_REDUCE_CTAS_PER_SM");
-    per_sm_env = e && atoi(e) > 0 ? atoi(e) : 0;
     const char *w = getenv("B200SHM_REDUCE_WAVES");
     if (w && atoi(w) > 0) waves = atoi(w);
+    per_sm_env = e && atoi(e) > 0 ? atoi(e) : 0;
   }
-  const int per_sm = per_sm_env ? per_sm_env : waves * resident_ctas(kernel);
-  return grid_for(lanes, 256, per_sm);
+  const uint64_t sms = (uint64_t)grid_sms();
+  int threads = 256;
+  while (threads > 64 && lanes < sms * (uint64_t)threads) threads >>= 1;
+  const int per_sm = per_sm_env ? per_sm_env : waves * resident_ctas((const void *)kernel);
+  kernel<<<grid_for(lanes, threads, per_sm), threads, 0, s>>>(a);
+  count_launch();
 }
 
-template <class K>
-void launch_one(K kernel, uint64_t lanes, cudaStream_t s, const RArgs &a) {
-  kernel<<<coop_grid((const void *)kernel, lanes), 256, 0, s>>>(a);
+/* the instance with or without edges */
+template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2, int MODE>
+void launch_edges(uint64_t lanes, cudaStream_t s, const RArgs &a) {
+  if constexpr (V > 1) {
+    if (a.nedge) {
+      launch_one(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, true>, lanes, s, a);
+      return;
+    }
+  }
+  launch_one(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, false>, lanes, s, a);
 }
 
-template <class T, int OP, int ORDER, int V, bool MM, int G>
-void launch_coop_g(int lvl, bool pow2, uint64_t lanes, cudaStream_t s, const RArgs &a) {
+/* leaves per lane n -> the instance */
+template <class T, int OP, int ORDER, int V, bool POW2, int MODE>
+void launch_tree(int n, uint64_t lanes, cudaStream_t s, const RArgs &a) {
+  constexpr int C16 = MODE == kPacks ? 16 : 0, C32 = MODE == kPacks ? 32 : 0;
+  switch (n) {
+  case 2: launch_edges<T, OP, ORDER, V, false, 2, POW2, MODE>(lanes, s, a); break;
+  case 4: launch_edges<T, OP, ORDER, V, false, 4, POW2, MODE>(lanes, s, a); break;
+  case 8: launch_edges<T, OP, ORDER, V, false, 8, POW2, MODE>(lanes, s, a); break;
+  case 16: launch_edges<T, OP, ORDER, V, false, C16, POW2, MODE>(lanes, s, a); break;
+  case 32: launch_edges<T, OP, ORDER, V, false, C32, POW2, MODE>(lanes, s, a); break;
+  default: launch_edges<T, OP, ORDER, V, false, 0, POW2, MODE>(lanes, s, a); break;
+  }
+}
+
+/* Lanes per column (log2), for `cols` columns over `leaves` leaves.
+ * Many columns: 2 lanes (1 where a lane would hold fewer than 8 leaves); for
+ * float trees as many as give each lane 32 leaves (2 to 8).  On the 64-PE
+ * workload G = 2 with 32 leaves per lane ran the f32 tree at 5.6-5.9 TB/s,
+ * G = 4 with 16 at 5.2-5.4 (a warp then reads 128 rather than 256
+ * consecutive bytes of each member per load).  Few columns: what counts is
+ * how many rounds of loads a lane makes in turn, so lanes are added while a
+ * lane holds more than 4 leaves and the columns are fewer than 128 per SM
+ * over G^2 (each doubling halves the run of each member that a warp reads,
+ * so it has to bring more each time: f32 SUM over 64 members of 1024 /
+ * 4096 / 16384 / 65536 elements ran 2.3 / 2.8 / 3.3 / 6.2 us at the 16 / 8 /
+ * 4 / 2 lanes this gives, and 4.3 / 5.5 / - / 6.0 at 2 before; at 16384 8
+ * lanes take 4.6 and 16 take 7.0).
+ * B200SHM_REDUCE_COOP sets the starting point (0 or 1 = one lane per
+ * column). */
+template <int ORDER>
+int lanes_log2(uint64_t cols, int leaves, bool wide) {
+  int G = wide ? 1 : 2; /* 16-byte elements: a chain of one lane per element */
+  if (ORDER != ORD_CHAIN) G = std::max(2, std::min(8, leaves / 32));
+  static const char *ec = getenv("B200SHM_REDUCE_COOP"); /* read once */
+  if (ec) G = std::max(1, std::min(8, atoi(ec)));
+  int lg = 31 - __builtin_clz((unsigned)G);
+  while (lg > 0 && (8 << lg) > leaves) lg--;
+  if (!ec)
+    while (lg < 4 && (4 << (lg + 1)) <= leaves &&
+           (cols << (2 * lg)) < (uint64_t)grid_sms() * 128)
+      lg++;
+  return lg;
+}
+
+template <class T, int OP, int ORDER, bool MM, int MODE>
+void run_mode(RArgs &a, cudaStream_t s) {
+  constexpr int V = MODE == kPacks && sizeof(T) < 16 ? (int)(16 / sizeof(T)) : 1;
+  const int P = a.P, leaves = ORDER == ORD_BUTTERFLY ? a.p2s : P;
+  const bool pow2 = (P & (P - 1)) == 0;
+  a.nvec = (a.N - a.head) / V;
+  a.nedge = (unsigned)(a.N - a.nvec * V);
+  /* splitting the members over lanes is exact for any-order ops, for
+   * butterflies, and for binomial trees over power-of-two teams */
+  constexpr bool any_order = ORDER == ORD_CHAIN && (std::is_integral<T>::value || MM);
+  const bool split = any_order || ORDER == ORD_BUTTERFLY || (ORDER == ORD_BINOMIAL && pow2);
+  a.lgG = split ? lanes_log2<ORDER>(a.nvec + a.nedge, leaves, sizeof(T) == 16) : 0;
+  const uint64_t lanes = std::max<uint64_t>(a.nvec + a.nedge, 1) << a.lgG;
   if constexpr (ORDER == ORD_CHAIN) {
-    launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 1, true>, lanes, s, a);
-  } else if constexpr (ORDER == ORD_BINOMIAL) { /* only power-of-two teams get here */
-    if (lvl == 1) launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 1, true>, lanes, s, a);
-    else if (lvl == 2) launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 2, true>, lanes, s, a);
-    else if (lvl == 4) launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 4, true>, lanes, s, a);
-    else launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 7, true>, lanes, s, a);
+    launch_edges<T, OP, ORDER, V, MM, 1, true, MODE>(lanes, s, a);
+  } else if constexpr (ORDER == ORD_BINOMIAL) {
+    if (pow2) launch_tree<T, OP, ORDER, V, true, MODE>(leaves >> a.lgG, lanes, s, a);
+    else if (P < 8) launch_edges<T, OP, ORDER, V, false, kRagged<3>, false, MODE>(lanes, s, a);
+    else if (P < 256) launch_edges<T, OP, ORDER, V, false, kRagged<8>, false, MODE>(lanes, s, a);
+    else launch_edges<T, OP, ORDER, V, false, kRagged<kMaxLevels>, false, MODE>(lanes, s, a);
   } else {
-    if (pow2) {
-      if (lvl == 1) launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 1, true>, lanes, s, a);
-      else if (lvl == 2) launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 2, true>, lanes, s, a);
-      else if (lvl == 4) launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 4, true>, lanes, s, a);
-      else launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 7, true>, lanes, s, a);
-    } else {
-      if (lvl == 1) launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 1, false>, lanes, s, a);
-      else if (lvl == 2) launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 2, false>, lanes, s, a);
-      else if (lvl == 4) launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 4, false>, lanes, s, a);
-      else launch_one(k_reduce_coop<T, OP, ORDER, V, G, MM, 7, false>, lanes, s, a);
-    }
+    if (pow2) launch_tree<T, OP, ORDER, V, true, MODE>(leaves >> a.lgG, lanes, s, a);
+    else launch_tree<T, OP, ORDER, V, false, MODE>(leaves >> a.lgG, lanes, s, a);
   }
 }
 
-template <class T, int OP, int ORDER, int V, bool MM>
-void launch_coop(int G, int lvl, bool pow2, uint64_t lanes, cudaStream_t s, const RArgs &a) {
-  switch (G) {
-  case 2: launch_coop_g<T, OP, ORDER, V, MM, 2>(lvl, pow2, lanes, s, a); break;
-  case 4: launch_coop_g<T, OP, ORDER, V, MM, 4>(lvl, pow2, lanes, s, a); break;
-  default: launch_coop_g<T, OP, ORDER, V, MM, 8>(lvl, pow2, lanes, s, a); break;
+template <class T, int OP, int ORDER, bool MM>
+int run(const RArgs &base, cudaStream_t s) {
+  if constexpr (ORDER != ORD_CHAIN) { /* one member: nothing to combine, a copy */
+    if (base.P == 1) return run<T, OP, ORD_CHAIN, false>(base, s);
   }
-}
-
-template <class T, int OP, int ORDER, bool MM, int LV>
-int run_lv(const RArgs &base, bool aligned, cudaStream_t s) {
-  constexpr int V = sizeof(T) >= 16 ? 1 : (int)(16 / sizeof(T));
-  constexpr int U = ORDER == ORD_CHAIN ? 8 : 4;
-  static int occ_pack = -1, occ_tail = -1;
   RArgs a = base;
-  uint64_t done = 0;
-  /* packs of several elements need 16-byte-aligned rows; a pack of one
-   * 16-byte element (complex double, long double) moves at any alignment,
-   * and its trees split over lanes too (long double SUM 1.52 -> 2.11 TB/s,
-   * PROD 2.20 -> 3.16 on 64 members x 2^18), while its chains stay one
-   * lane per element (long double MAX split over lanes: 2.56 -> 2.11) */
-  if ((V > 1 ? aligned : ORDER != ORD_CHAIN) && done < base.N) {
-    a.e_begin = done;
-    a.nvec = (base.N - done) / V;
-    if (a.nvec) {
-      /* warp-cooperative split of the leaves is exact for any-order ops,
-       * for butterflies, and for binomial trees over power-of-two teams.
-       * G lanes per column: 2 for chains; for float trees as many as give
-       * each lane 32 leaves (2 to 8).  On the 64-PE workload G = 2 with
-       * 32 leaves per lane ran the f32 tree at 5.6-5.9 TB/s, G = 4 with 16
-       * at 5.2-5.4 (a warp then reads 128 rather than 256 consecutive bytes
-       * of each member per load).  B200SHM_REDUCE_COOP overrides (0 or 1 =
-       * one lane per column). */
-      constexpr bool any_order = ORDER == ORD_CHAIN && (std::is_integral<T>::value || MM);
-      const int nleaves = ORDER == ORD_BUTTERFLY ? base.p2s : base.P;
-      const bool splittable = any_order || ORDER == ORD_BUTTERFLY ||
-                              (ORDER == ORD_BINOMIAL && (base.P & (base.P - 1)) == 0);
-      /* float trees: 32 leaves per lane (four 8-leaf chunks, two slots),
-       * so G = 2 at 64 leaves; chains: G = 2 */
-      int G = 2;
-      if constexpr (ORDER != ORD_CHAIN) G = std::max(2, std::min(8, nleaves / 32));
-      static const char *ec = getenv("B200SHM_REDUCE_COOP"); /* read once */
-      if (ec) G = atoi(ec);
-      if (G < 1) G = 1;
-      if (G > 32) G = 32;
-      if (G > 8) G = 8;
-      G = 1 << (31 - __builtin_clz((unsigned)G)); /* power of two */
-      while (G > 1 && G * 8 > nleaves) G >>= 1;
-      if constexpr (ORDER != ORD_CHAIN || any_order) {
-        if (splittable && G >= 2) {
-          const uint64_t lanes = a.nvec * (uint64_t)G;
-          const int chunks = nleaves / G / 8; /* tree chunks per lane */
-          const bool pow2 = ORDER != ORD_BUTTERFLY || base.P == base.p2s;
-          launch_coop<T, OP, ORDER, V, MM>(G, ORDER == ORD_CHAIN ? 1 : chunks <= 1 ? 1 : chunks == 2 ? 2
-                                                 : chunks == 4 ? 4 : 7,
-                                           pow2, lanes, s, a);
-          count_launch();
-          done += a.nvec * V;
-        }
-      }
-      if (done < base.N && a.e_begin == done) {
-        auto k = k_reduce<T, OP, ORDER, V, U, MM, LV>;
-        k<<<reduce_grid(k, occ_pack, a.nvec, 256), 256, 0, s>>>(a);
-        count_launch();
-        done += a.nvec * V;
-      }
-    }
-  }
-  if (done < base.N) {
-    a.e_begin = done;
-    a.nvec = base.N - done;
-    auto k = k_reduce<T, OP, ORDER, 1, U, MM, LV>;
-    k<<<reduce_grid(k, occ_tail, a.nvec, 256), 256, 0, s>>>(a);
-    count_launch();
+  const uint64_t steps = a.P > 1 ? a.sstep | a.dstep : 0;
+  const uintptr_t sp = (uintptr_t)a.src, dp = (uintptr_t)a.dst;
+  a.head = 0;
+  if (!MM || a.p2s <= kExactLeaves) a.fix_list = nullptr;
+  if (((sp ^ dp) & 15) == 0 && (steps & 15) == 0 && dp % sizeof(T) == 0) {
+    /* the packs begin at a 128-byte line of the dest, so that warps do not
+     * share lines (vectors shorter than a few lines: at the 16-byte grid) */
+    const uintptr_t grid = sizeof(T) < 16 && a.N * sizeof(T) >= 4096 ? 128 : 16;
+    a.head = (unsigned)std::min<uint64_t>((grid - (dp & (grid - 1))) % grid / sizeof(T), a.N);
+    run_mode<T, OP, ORDER, MM, kPacks>(a, s);
+  } else if (sizeof(T) < 16 && ((sp | dp | steps) % sizeof(T)) == 0) {
+    run_mode<T, OP, ORDER, MM, sizeof(T) < 16 ? kElements : kBytes>(a, s);
+  } else {
+    run_mode<T, OP, ORDER, MM, kBytes>(a, s);
   }
   if constexpr (MM) {
+    if (a.fix_list == nullptr) return B200SHM_OK;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * grid_sms());
     cfg.blockDim = dim3(256);
@@ -587,52 +679,41 @@ int run_lv(const RArgs &base, bool aligned, cudaStream_t s) {
   return B200SHM_OK;
 }
 
-template <class T, int OP, int ORDER, bool MM>
-int run(const RArgs &base, bool aligned, cudaStream_t s) {
-  if constexpr (ORDER == ORD_CHAIN) {
-    return run_lv<T, OP, ORDER, MM, 1>(base, aligned, s);
-  } else {
-    const int leaves = ORDER == ORD_BUTTERFLY ? base.p2s : base.P;
-    if (leaves < (1 << 8)) return run_lv<T, OP, ORDER, MM, 8>(base, aligned, s);
-    return run_lv<T, OP, ORDER, MM, kMaxLevels>(base, aligned, s);
-  }
-}
-
 template <class T, int OP>
-int run_float(const RArgs &a, bool aligned, cudaStream_t s) {
+int run_float(const RArgs &a, cudaStream_t s) {
   if constexpr (OP == B200SHM_MIN || OP == B200SHM_MAX) {
     /* the deferred count is zero here: the previous replay cleared it */
-    return run<T, OP, ORD_CHAIN, true>(a, aligned, s);
+    return run<T, OP, ORD_CHAIN, true>(a, s);
   } else {
     switch (a.algo) {
-    case B200SHM_LINEAR: return run<T, OP, ORD_CHAIN, false>(a, aligned, s);
-    case B200SHM_BINOMIAL: return run<T, OP, ORD_BINOMIAL, false>(a, aligned, s);
-    default: return run<T, OP, ORD_BUTTERFLY, false>(a, aligned, s);
+    case B200SHM_LINEAR: return run<T, OP, ORD_CHAIN, false>(a, s);
+    case B200SHM_BINOMIAL: return run<T, OP, ORD_BINOMIAL, false>(a, s);
+    default: return run<T, OP, ORD_BUTTERFLY, false>(a, s);
     }
   }
 }
 
 template <class T, int OP>
-int run_cplx(const RArgs &a, bool aligned, cudaStream_t s) {
+int run_cplx(const RArgs &a, cudaStream_t s) {
   switch (a.algo) {
-  case B200SHM_LINEAR: return run<T, OP, ORD_CHAIN, false>(a, aligned, s);
-  case B200SHM_BINOMIAL: return run<T, OP, ORD_BINOMIAL, false>(a, aligned, s);
-  default: return run<T, OP, ORD_BUTTERFLY, false>(a, aligned, s);
+  case B200SHM_LINEAR: return run<T, OP, ORD_CHAIN, false>(a, s);
+  case B200SHM_BINOMIAL: return run<T, OP, ORD_BINOMIAL, false>(a, s);
+  default: return run<T, OP, ORD_BUTTERFLY, false>(a, s);
   }
 }
 
 /* Integer ops other than MIN/MAX give the same bits on signed and unsigned
  * views, so they run on the unsigned type of the same width. */
 template <class S, class U>
-int run_int(int op, const RArgs &a, bool aligned, cudaStream_t s) {
+int run_int(int op, const RArgs &a, cudaStream_t s) {
   switch (op) {
-  case B200SHM_AND: return run<U, B200SHM_AND, ORD_CHAIN, false>(a, aligned, s);
-  case B200SHM_OR: return run<U, B200SHM_OR, ORD_CHAIN, false>(a, aligned, s);
-  case B200SHM_XOR: return run<U, B200SHM_XOR, ORD_CHAIN, false>(a, aligned, s);
-  case B200SHM_MIN: return run<S, B200SHM_MIN, ORD_CHAIN, false>(a, aligned, s);
-  case B200SHM_MAX: return run<S, B200SHM_MAX, ORD_CHAIN, false>(a, aligned, s);
-  case B200SHM_SUM: return run<U, B200SHM_SUM, ORD_CHAIN, false>(a, aligned, s);
-  default: return run<U, B200SHM_PROD, ORD_CHAIN, false>(a, aligned, s);
+  case B200SHM_AND: return run<U, B200SHM_AND, ORD_CHAIN, false>(a, s);
+  case B200SHM_OR: return run<U, B200SHM_OR, ORD_CHAIN, false>(a, s);
+  case B200SHM_XOR: return run<U, B200SHM_XOR, ORD_CHAIN, false>(a, s);
+  case B200SHM_MIN: return run<S, B200SHM_MIN, ORD_CHAIN, false>(a, s);
+  case B200SHM_MAX: return run<S, B200SHM_MAX, ORD_CHAIN, false>(a, s);
+  case B200SHM_SUM: return run<U, B200SHM_SUM, ORD_CHAIN, false>(a, s);
+  default: return run<U, B200SHM_PROD, ORD_CHAIN, false>(a, s);
   }
 }
 
