@@ -11,14 +11,19 @@
  * is one copy kernel that moves every byte once from its source slice to
  * its final place: no rounds, no intermediate copies, no rotation.
  *
- * Copies run in 16-byte vectors when every base offset and size is a
- * multiple of 16, else in bytes (or elements for the strided form).
+ * fcollect, collect, broadcast and alltoall write each dest row as the
+ * aligned 16-byte vectors it spans, whatever the offsets and block sizes:
+ * a vector is cut out of the source blocks that meet in it (copy_core.cuh),
+ * and only the two vectors at the row's ends are written in bytes.  The
+ * strided form copies elements.
  */
 #include <stdint.h>
 #include <stdlib.h>
+#include <string.h>
 
 #include <vector>
 
+#include "copy_core.cuh"
 #include "internal.cuh"
 
 namespace b200 {
@@ -27,6 +32,14 @@ namespace {
 __device__ __forceinline__ uint4 ld16(const char *p) {
   uint4 u;
   asm("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+      : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
+      : "l"(p));
+  return u;
+}
+/* a vector the next lane reads too */
+__device__ __forceinline__ uint4 ld16l1(const char *p) {
+  uint4 u;
+  asm("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];"
       : "=r"(u.x), "=r"(u.y), "=r"(u.z), "=r"(u.w)
       : "l"(p));
   return u;
@@ -45,27 +58,144 @@ __device__ __forceinline__ void st16cs(char *p, uint4 u) {
                : "memory");
 }
 
-/* fcollect: member j's dest[k*nbytes + b] = member k's src[b].
- * blockIdx.y = source member k; each thread reads one vector of k's
- * source once and writes it into every member's dest (streaming stores:
- * 5.99 against 5.92 TB/s with write-back stores, and 5.93 with each CTA
- * starting at its own member, on 128 members x 32 KiB). */
-template <bool VEC>
-__global__ void __launch_bounds__(256) k_fcollect(const char *src0, char *dst0, uint64_t step,
-                                                  int P, uint64_t nbytes) {
-  const int k = blockIdx.y;
-  const char *src = src0 + (uint64_t)k * step;
-  char *dst = dst0 + (uint64_t)k * nbytes;
-  const uint64_t n = VEC ? nbytes / 16 : nbytes;
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
-       v += (uint64_t)gridDim.x * blockDim.x) {
-    if constexpr (VEC) {
-      const uint4 u = ld16(src + v * 16);
-      for (int j = 0; j < P; j++) st16cs(dst + (uint64_t)j * step + v * 16, u);
-    } else {
-      const char c = src[v];
-      for (int j = 0; j < P; j++) dst[(uint64_t)j * step + v] = c;
+/* The bytes [i0, i1) of a vector, 16 bytes at virtual address s of which the
+ * first n1 bytes (and none below i0) come from there, the others from c on,
+ * counted from the vector's byte 0 too.  All loads are issued together. */
+__device__ __forceinline__ uint4 meet16(const char *s, const char *c, int i0, int n1, int i1) {
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4 lo = zero, hi = zero, clo = zero, chi = zero;
+  const int sh = (int)((uintptr_t)s & 15), csh = (int)((uintptr_t)c & 15);
+  if (sh + i0 < 16) lo = ld16l1(s - sh);
+  if (sh + n1 > 16) hi = ld16l1(s - sh + 16);
+  if (n1 < i1) {
+    if (csh + n1 < 16) clo = ld16l1(c - csh);
+    if (csh + i1 > 16) chi = ld16l1(c - csh + 16);
+  }
+  return join16(cut16(lo, hi, sh), cut16(clo, chi, csh), n1);
+}
+
+/* What a dest row concatenates: P blocks, block k read at src0 + k*step. */
+struct Even { /* of B bytes each */
+  uint64_t B;
+  __device__ __forceinline__ int find(uint64_t x, int, uint64_t *b) const {
+    const uint64_t k = x / B;
+    *b = x - k * B;
+    return (int)k;
+  }
+  __device__ __forceinline__ uint64_t size(int) const { return B; }
+};
+/* of uneven sizes: pre[k] = the row position of block k, pre[P] = the row's
+ * length.  The table is the kernel's parameter (N entries at most), read
+ * through the constant cache; N = 0: a table in device memory. */
+template <int N>
+struct Uneven {
+  uint64_t pre[N];
+};
+template <>
+struct Uneven<0> {
+  const uint64_t *pre;
+};
+template <int N>
+struct Table {
+  const Uneven<N> &t;
+  /* the last k with pre[k] <= x: x is below the row's length, so that
+   * block is not empty */
+  __device__ __forceinline__ int find(uint64_t x, int P, uint64_t *b) const {
+    int lo = 0, hi = P;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) / 2;
+      if (t.pre[mid] <= x)
+        lo = mid;
+      else
+        hi = mid;
     }
+    *b = x - t.pre[lo];
+    return lo;
+  }
+  __device__ __forceinline__ uint64_t size(int k) const { return t.pre[k + 1] - t.pre[k]; }
+};
+__device__ __forceinline__ Even blocks(const Even &e) { return e; }
+template <int N>
+__device__ __forceinline__ Table<N> blocks(const Uneven<N> &t) {
+  return Table<N>{t};
+}
+
+/* fcollect, collect and broadcast: every member's dest row is the same
+ * `len` bytes, the blocks one after the other (fcollect.c:370-403,
+ * collect.c:35-591).  One thread per 16-byte vector of the row: it puts the
+ * vector together once and writes it into the members of its blockIdx.y
+ * (all but `skip`).  Bound by the writes, P per vector read; streaming
+ * stores, since this kernel does not read them again.  128 members x 32 KiB:
+ * 92.4 us with one pass per source member and six CTAs an SM, 80.3 now (6.7
+ * TB/s); x 32764 bytes, then 4-byte words: 274 -> 81.4; collect of 64 members
+ * x 32 KiB on average, 4-byte words and an uploaded table: 40.7 -> 24.5. */
+template <class BLK>
+__global__ void __launch_bounds__(256, 6) k_spread(const char *src0, char *dst0, uint64_t step,
+                                                int P, uint64_t len, int nblk, int mpc, int skip,
+                                                const __grid_constant__ BLK prm) {
+  const auto blk = blocks(prm);
+  const int a = (int)((uintptr_t)dst0 & 15); /* the row begins at byte a of vector 0 */
+  const int64_t x0 = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 16 - a;
+  const int i0 = x0 < 0 ? a : 0;
+  const int i1 = (int64_t)len - x0 < 16 ? (int)((int64_t)len - x0) : 16;
+  const int j0 = blockIdx.y * mpc, j1 = j0 + mpc < P ? j0 + mpc : P;
+  uint4 u = make_uint4(0, 0, 0, 0);
+  uint64_t left = 0;
+  const char *s = nullptr;
+  int k = 0;
+  if (i1 > i0) {
+    uint64_t b;
+    k = blk.find((uint64_t)(x0 + i0), nblk, &b);
+    left = blk.size(k) - b;
+    s = src0 + (uint64_t)k * step + b;
+  }
+  /* one way for the whole warp, so that its loads are issued together */
+  const bool inside = __all_sync(~0u, i1 <= i0 || (left >= 16 && i1 - i0 == 16));
+  if (i1 > i0) {
+    if (inside) {
+      const unsigned sh = (unsigned)(uintptr_t)s & 15u;
+      u = ld16l1(s - sh);
+      if (sh) u = cut16(u, ld16l1(s - sh + 16), sh);
+    } else {
+      const int n1 = left < (uint64_t)(i1 - i0) ? i0 + (int)left : i1;
+      if (n1 == i1 || blk.size(k + 1) >= (uint64_t)(i1 - n1)) {
+        u = meet16(s - i0, src0 + (uint64_t)(k + 1) * step - n1, i0, n1, i1);
+      } else { /* small blocks, more than two of them: byte by byte */
+        unsigned w[4] = {0, 0, 0, 0};
+        for (int i = i0; i < i1; i++) {
+          while (left == 0) { /* the next block with a byte */
+            left = blk.size(++k);
+            s = src0 + (uint64_t)k * step;
+          }
+          const unsigned c = (unsigned)(unsigned char)*s << (8 * (i & 3));
+#pragma unroll
+          for (int q = 0; q < 4; q++) w[q] |= i >> 2 == q ? c : 0;
+          s++;
+          left--;
+        }
+        u = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    }
+    if (i1 - i0 == 16) {
+      char *d = dst0 + x0 + (uint64_t)j0 * step;
+      for (int j = j0; j < j1; j++, d += step)
+        if (j != skip) st16cs(d, u);
+    }
+  }
+  /* the row's ends, in bytes: the members over the warp's lanes */
+  unsigned ends = __ballot_sync(~0u, i1 > i0 && i1 - i0 < 16);
+  while (ends) {
+    const int from = __ffs(ends) - 1;
+    ends &= ends - 1;
+    const unsigned w[4] = {__shfl_sync(~0u, u.x, from), __shfl_sync(~0u, u.y, from),
+                           __shfl_sync(~0u, u.z, from), __shfl_sync(~0u, u.w, from)};
+    const int e0 = __shfl_sync(~0u, i0, from), e1 = __shfl_sync(~0u, i1, from);
+    char *d = dst0 + __shfl_sync(~0u, x0, from);
+    for (int j = j0 + (int)(threadIdx.x & 31); j < j1; j += 32)
+      if (j != skip)
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+          if (i >= e0 && i < e1) d[(uint64_t)j * step + i] = (char)(w[i >> 2] >> (8 * (i & 3)));
   }
 }
 
@@ -165,60 +295,154 @@ __global__ void __launch_bounds__(256) k_fcollect_bulk(const char *src0, char *d
   __syncthreads();
 }
 
-/* collect: member k contributes sizes[k] bytes; member j's
- * dest[prefix[k] + b] = member k's src[b] (collect.c:35-591: the
- * contributions concatenated in member order).  blockIdx.y = source member
- * k; each thread reads one word of k's contribution once and writes it
- * into every member's dest.  W is a width every offset and size divides. */
-template <class W>
-__global__ void __launch_bounds__(256) k_collect(const char *src0, char *dst0, uint64_t step,
-                                                 int P, const uint64_t *sizes,
-                                                 const uint64_t *prefix) {
-  const int k = blockIdx.y;
-  const W *src = (const W *)(src0 + (uint64_t)k * step);
-  char *dst = dst0 + prefix[k];
-  const uint64_t n = sizes[k] / sizeof(W);
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
-       v += (uint64_t)gridDim.x * blockDim.x) {
-    const W u = src[v];
-    for (int j = 0; j < P; j++) ((W *)(dst + (uint64_t)j * step))[v] = u;
-  }
-}
-
 /* alltoall: member j's dest[k*B + b] = member k's src[j*B + b].
- * Pairs k*P + j are spread over blockIdx.y (grid-stride when there are more
- * pairs than the grid's y extent); blockIdx.x strides over the block. */
-template <bool VEC>
-__global__ void __launch_bounds__(256) k_alltoall(const char *src0, char *dst0, uint64_t step,
-                                                  int P, uint64_t B) {
-  const uint64_t pairs = (uint64_t)P * (uint64_t)P;
-  const uint64_t n = VEC ? B / 16 : B;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-  for (uint64_t pr = blockIdx.y; pr < pairs; pr += gridDim.y) {
-    const uint64_t k = pr / (uint64_t)P, j = pr % (uint64_t)P;
-    const char *src = src0 + k * step + j * B;
-    char *dst = dst0 + j * step + k * B;
-    uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if constexpr (VEC) {
-      /* four vectors in flight per thread */
-      for (; v + 3 * stride < n; v += 4 * stride) {
-        uint4 u0 = ld16(src + v * 16), u1 = ld16(src + (v + stride) * 16);
-        uint4 u2 = ld16(src + (v + 2 * stride) * 16), u3 = ld16(src + (v + 3 * stride) * 16);
-        st16(dst + v * 16, u0);
-        st16(dst + (v + stride) * 16, u1);
-        st16(dst + (v + 2 * stride) * 16, u2);
-        st16(dst + (v + 3 * stride) * 16, u3);
-      }
-      for (; v < n; v += stride) st16(dst + v * 16, ld16(src + v * 16));
-    } else {
-      for (; v < n; v += stride) dst[v] = src[v];
+ * A CTA writes 256 * U vectors, its tile, of one dest row (blockIdx.y,
+ * striding where a team has more rows than the grid's y extent). */
+
+/* Where the bytes of a tile come from: the tile begins at position x0 of
+ * the row, byte b0 of block k0.  It crosses at most one block end when B is
+ * larger than it; otherwise `recip` = floor(2^32 / B) + 1 and
+ * umulhi(position, recip) is the block exactly: positions stay at or below
+ * B + TILE <= 2^15 and B <= 2^14, so the product's error, at most position
+ * / 2^32, is below 1 / B. */
+template <int TILE>
+struct BlockWalk {
+  int64_t x0, b0;
+  uint64_t k0;
+  int lim; /* the tile offset of block k0's end, at most TILE */
+  uint64_t jump; /* from a block's end to the next block's first byte */
+  unsigned B32, recip;
+  __device__ __forceinline__ BlockWalk(int a, uint64_t step, uint64_t B, unsigned r) {
+    x0 = (int64_t)blockIdx.x * TILE - a;
+    k0 = x0 > 0 ? (uint64_t)x0 / B : 0;
+    b0 = x0 - (int64_t)(k0 * B);
+    lim = (int64_t)B - b0 < TILE ? (int)((int64_t)B - b0) : TILE;
+    jump = step - B;
+    B32 = (unsigned)B;
+    recip = r;
+  }
+  /* the source of the byte at tile offset t, from that of offset 0 in k0;
+   * *rem: bytes left in its block, or in the tile where that is less */
+  __device__ __forceinline__ const char *at(const char *col, int t, int *rem) const {
+    if (recip) {
+      const unsigned bi = (unsigned)((int)b0 + t), q = __umulhi(bi, recip);
+      *rem = (int)((q + 1) * B32 - bi);
+      return col + t + q * jump;
+    }
+    const bool past = t >= lim;
+    *rem = past ? TILE - t : lim - t;
+    return col + t + (past ? jump : 0);
+  }
+};
+
+/* Blocks of whole aligned vectors, neighbouring threads on neighbouring
+ * dest vectors whatever the block size (one block pair a CTA left most
+ * threads of small blocks idle).  128 members x 64 KiB: 333 -> 318 us (6.7
+ * TB/s); x 4 KiB: 37.0 -> 22.3; x 1008 bytes: 8.35 -> 7.7. */
+template <int U>
+__global__ void __launch_bounds__(256, 4) k_alltoall(const char *src0, char *dst0, uint64_t step,
+                                                     int P, uint64_t B, unsigned recip) {
+  const BlockWalk<4096 * U> w(0, step, B, recip);
+  const int64_t end = (int64_t)((uint64_t)P * B) - w.x0;
+  for (uint64_t j = blockIdx.y; j < (uint64_t)P; j += gridDim.y) {
+    char *row = dst0 + j * step + w.x0;
+    const char *col = src0 + j * B + w.k0 * step + w.b0;
+    uint4 x[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int t = ((int)threadIdx.x + u * 256) * 16;
+      int rem;
+      const char *s = w.at(col, t, &rem);
+      if (t < end) x[u] = ld16(s);
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int t = ((int)threadIdx.x + u * 256) * 16;
+      if (t < end) st16(row + t, x[u]);
     }
   }
 }
 
-/* alltoall of small blocks (fewer words per pair than a CTA has threads):
- * one thread per word of the flattened [pair][word] space, so a CTA spans
- * many pairs instead of idling most of its threads on one. */
+/* 16 bytes from byte 4 * Q + bits / 8 of lo, hi */
+template <int Q>
+__device__ __forceinline__ uint4 cut_at(uint4 lo, uint4 hi, unsigned bits) {
+  const unsigned w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+  return make_uint4(
+      __funnelshift_r(w[Q], w[Q + 1], bits), __funnelshift_r(w[Q + 1], w[Q + 2], bits),
+      __funnelshift_r(w[Q + 2], w[Q + 3], bits), __funnelshift_r(w[Q + 3], w[Q + 4], bits));
+}
+/* A lane's vectors of a warp whose bytes lie in one block: 512 apart at
+ * the 16-byte aligned d, from s at the shift 4 * Q + bits / 8. */
+template <int U, int Q>
+__device__ __forceinline__ void cut_run(char *d, const char *s, unsigned bits) {
+  uint4 lo[U], hi[U];
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    lo[u] = ld16l1(s + u * 512);
+    hi[u] = Q == 0 && bits == 0 ? lo[u] : ld16l1(s + u * 512 + 16);
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++) st16(d + u * 512, cut_at<Q>(lo[u], hi[u], bits));
+}
+
+/* Any offsets and blocks of 16 bytes or more: each aligned dest vector is
+ * cut out of two neighbouring source vectors, the second of which is the
+ * next lane's first and comes from L1.  A warp writes 32 * U vectors in a
+ * row.  What bounds it off the memory is the instructions per vector: where
+ * the warp's bytes lie in one block, the shift is the warp's, the word part
+ * of it a branch and the rest one funnel shift a word; the warps in whose
+ * bytes a block ends look for the block of each vector.  (The same search
+ * for every vector took 163 instructions each and 457 us for 128 members x
+ * 65532 bytes.)  Against one word of the blocks' common width a thread: 128
+ * members x 65532 bytes 1800 -> 321 us (6.7 TB/s), x 9999 289 -> 59.5, x 1004
+ * 23.6 -> 12.4. */
+template <int U>
+__global__ void __launch_bounds__(256, U > 2 ? 4 : 6)
+    k_alltoall_shift(const char *src0, char *dst0, uint64_t step, int P, uint64_t B,
+                     unsigned recip) {
+  const int a = (int)((uintptr_t)dst0 & 15);
+  const BlockWalk<4096 * U> w(a, step, B, recip);
+  const int64_t end = (int64_t)((uint64_t)P * B) - w.x0;
+  const int lane = (int)(threadIdx.x & 31), tw = (int)(threadIdx.x >> 5) * 512 * U;
+  if (tw >= end) return;
+  for (uint64_t j = blockIdx.y; j < (uint64_t)P; j += gridDim.y) {
+    char *row = dst0 + j * step + w.x0;
+    const char *col = src0 + j * B + w.k0 * step + w.b0;
+    int rem;
+    const char *s = w.at(col, tw, &rem);
+    if (w.x0 + tw >= 0 && tw + 512 * U <= end && rem >= 512 * U) {
+      const unsigned sh = (unsigned)(uintptr_t)s & 15u, bits = (sh & 3) * 8;
+      char *d = row + tw + lane * 16;
+      s += lane * 16 - (int)sh;
+      switch (sh >> 2) {
+      case 0: cut_run<U, 0>(d, s, bits); break;
+      case 1: cut_run<U, 1>(d, s, bits); break;
+      case 2: cut_run<U, 2>(d, s, bits); break;
+      default: cut_run<U, 3>(d, s, bits);
+      }
+      continue;
+    }
+#pragma unroll 1
+    for (int u = 0; u < U; u++) {
+      const int t = tw + u * 512 + lane * 16;
+      if (w.x0 + t >= 0 && t + 16 <= end) {
+        s = w.at(col, t, &rem);
+        st16(row + t, meet16(s, s + w.jump, 0, rem < 16 ? rem : 16, 16));
+      } else if (t < end) { /* the row's ends: byte by byte */
+#pragma unroll 1
+        for (int i = 0; i < 16; i++) {
+          const int64_t y = w.x0 + t + i;
+          if (y < 0 || t + i >= end) continue;
+          const uint64_t k = (uint64_t)y / B;
+          row[t + i] = src0[j * B + k * step + ((uint64_t)y - k * B)];
+        }
+      }
+    }
+  }
+}
+
+/* alltoall of blocks of less than 16 bytes: one thread per word of the
+ * flattened [pair][word] space. */
 template <class W>
 __global__ void __launch_bounds__(256) k_alltoall_flat(const char *src0, char *dst0,
                                                        uint64_t step, int P, uint64_t nw) {
@@ -282,28 +506,9 @@ __global__ void __launch_bounds__(256) k_alltoalls_bytes(const char *src0, char 
   }
 }
 
-/* broadcast: every member but the root gets the root's source */
-template <bool VEC>
-__global__ void __launch_bounds__(256) k_broadcast(const char *src, char *dst0, uint64_t step,
-                                                   int P, int root, uint64_t nbytes) {
-  const uint64_t n = VEC ? nbytes / 16 : nbytes;
-  for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
-       v += (uint64_t)gridDim.x * blockDim.x) {
-    if constexpr (VEC) {
-      const uint4 u = ld16(src + v * 16);
-      for (int j = 0; j < P; j++)
-        if (j != root) st16(dst0 + (uint64_t)j * step + v * 16, u);
-    } else {
-      const char c = src[v];
-      for (int j = 0; j < P; j++)
-        if (j != root) dst0[(uint64_t)j * step + v] = c;
-    }
-  }
-}
-
 /* Pairs of an all-to-all beyond this many loop over blockIdx.y. */
 constexpr uint64_t kMaxGridY = 65535;
-/* Blocks of fewer words than this per pair take the flattened kernels. */
+/* Strided blocks of fewer elements than this per pair take the flattened kernel. */
 constexpr uint64_t kFlatWords = 64;
 
 /* CTAs along x for a per-pair / per-member extent of n work items, so that
@@ -314,6 +519,33 @@ unsigned x_blocks(uint64_t n, uint64_t ypairs, uint64_t want) {
   if (cap < 1) cap = 1;
   if (per > cap) per = cap;
   return (unsigned)(per < 1 ? 1 : per);
+}
+
+/* Launch k_spread over a row of len bytes: rows of few vectors split their
+ * members over more CTAs, so that the grid fills the SMs. */
+template <class BLK>
+void spread(const char *src, char *dst, uint64_t step, int P, uint64_t len, int nblk, int skip,
+            const BLK &blk, cudaStream_t s) {
+  const uint64_t tiles = (((uintptr_t)dst & 15) + len + 4095) / 4096;
+  uint64_t split = (8ull * st().sm_count + tiles - 1) / tiles;
+  if (split > (uint64_t)P) split = (uint64_t)P;
+  const int mpc = (int)((P + split - 1) / split);
+  dim3 grid((unsigned)tiles, (unsigned)((P + mpc - 1) / mpc));
+  /* Long rows run two CTAs an SM, by a claim on shared memory: fewer rows
+   * are written at a time, which DRAM likes better (128 members x 32 KiB:
+   * 80.5 us with two, 82.5 with three, 85.9 with six).  Rows of fewer
+   * vectors want the CTAs (32 members x 32 KiB: 8.3 us with six, 9.4 with
+   * two). */
+  constexpr int kHalfSm = 100000;
+  size_t smem = 0;
+  if (tiles >= 1024) {
+    static const bool ok = cudaFuncSetAttribute(k_spread<BLK>,
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                kHalfSm) == cudaSuccess;
+    if (ok) smem = kHalfSm;
+  }
+  k_spread<BLK><<<grid, 256, smem, s>>>(src, dst, step, P, len, nblk, mpc, skip, blk);
+  count_launch();
 }
 
 }  // namespace
@@ -331,7 +563,6 @@ int fcollect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
   if (P > 65535) return fail(B200SHM_ERR_UNSUPPORTED, "fcollect: more than 65535 members");
   Members m = members(pe_start, pe_stride, P);
   const bool vec = ((src_off | dest_off | nbytes | m.step) & 15u) == 0;
-  const uint64_t n = vec ? nbytes / 16 : nbytes;
   static const bool bulk = getenv("B200SHM_FCOLLECT_BULK") && atoi(getenv("B200SHM_FCOLLECT_BULK")) > 0;
   if (vec && bulk) { /* the staged form, selected for measurement */
     const uint64_t ntiles = (nbytes + kFcBulkTile - 1) / kFcBulkTile;
@@ -342,12 +573,8 @@ int fcollect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
     count_launch();
     return B200SHM_OK;
   }
-  dim3 grid(x_blocks(n, P, 8ull * st().sm_count * 4), P);
-  if (vec)
-    k_fcollect<true><<<grid, 256, 0, s>>>(m.first + src_off, m.first + dest_off, m.step, P, nbytes);
-  else
-    k_fcollect<false><<<grid, 256, 0, s>>>(m.first + src_off, m.first + dest_off, m.step, P, nbytes);
-  count_launch();
+  spread(m.first + src_off, m.first + dest_off, m.step, P, nbytes * (uint64_t)P, P, -1,
+         Even{nbytes}, s);
   return B200SHM_OK;
 }
 
@@ -357,40 +584,43 @@ int collect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint64
   if (rc) return rc;
   if (!nbytes) return fail(B200SHM_ERR_ARG, "collect: null size array");
   if (P > 65535) return fail(B200SHM_ERR_UNSUPPORTED, "collect: more than 65535 members");
-  std::vector<uint64_t> host(2 * (size_t)P);
-  uint64_t total = 0, biggest = 0, bits = 0;
+  std::vector<uint64_t> pre((size_t)P + 1);
+  uint64_t total = 0, biggest = 0;
   for (int k = 0; k < P; k++) {
     if (nbytes[k] > st().slice || total + nbytes[k] > st().slice)
       return fail(B200SHM_ERR_ARG, "collect: contributions larger than a heap slice");
-    host[k] = nbytes[k];
-    host[P + k] = total;
+    pre[k] = total;
     total += nbytes[k];
     if (nbytes[k] > biggest) biggest = nbytes[k];
-    bits |= nbytes[k];
   }
+  pre[P] = total;
   if ((rc = check_extent(src_off, biggest, "collect source"))) return rc;
   if ((rc = check_extent(dest_off, total, "collect dest"))) return rc;
   if (overlaps(dest_off, total, src_off, biggest))
     return fail(B200SHM_ERR_ARG, "collect: dest and source overlap");
   if (total == 0) return B200SHM_OK;
   Members m = members(pe_start, pe_stride, P);
-  bits |= src_off | dest_off | m.step;
-  const uint64_t w = bits & 15 ? (bits & 7 ? (bits & 3 ? 1 : 4) : 8) : 16;
-  uint64_t *dev = nullptr;
-  B200_CK(cudaMallocAsync((void **)&dev, host.size() * sizeof(uint64_t), s));
-  B200_CK(cudaMemcpyAsync(dev, host.data(), host.size() * sizeof(uint64_t),
-                          cudaMemcpyHostToDevice, s));
-  dim3 grid(x_blocks(biggest / w, P, 8ull * st().sm_count * 4), P);
   const char *src = m.first + src_off;
   char *dst = m.first + dest_off;
-  switch (w) {
-  case 16: k_collect<uint4><<<grid, 256, 0, s>>>(src, dst, m.step, P, dev, dev + P); break;
-  case 8: k_collect<unsigned long long><<<grid, 256, 0, s>>>(src, dst, m.step, P, dev, dev + P); break;
-  case 4: k_collect<unsigned><<<grid, 256, 0, s>>>(src, dst, m.step, P, dev, dev + P); break;
-  default: k_collect<unsigned char><<<grid, 256, 0, s>>>(src, dst, m.step, P, dev, dev + P); break;
+  /* The table of positions as a kernel parameter (64 members x 32 KiB on
+   * average: 46 us with an allocation, an upload and a free around the
+   * kernel); teams too large for one keep it in device memory. */
+  auto by_value = [&](auto blk) {
+    memcpy(blk.pre, pre.data(), pre.size() * sizeof(uint64_t));
+    spread(src, dst, m.step, P, total, P, -1, blk, s);
+  };
+  if (P < 136) {
+    by_value(Uneven<136>{});
+  } else if (P < 1032) {
+    by_value(Uneven<1032>{});
+  } else {
+    uint64_t *dev = nullptr;
+    B200_CK(cudaMallocAsync((void **)&dev, pre.size() * sizeof(uint64_t), s));
+    B200_CK(cudaMemcpyAsync(dev, pre.data(), pre.size() * sizeof(uint64_t),
+                            cudaMemcpyHostToDevice, s));
+    spread(src, dst, m.step, P, total, P, -1, Uneven<0>{dev}, s);
+    B200_CK(cudaFreeAsync(dev, s));
   }
-  count_launch();
-  B200_CK(cudaFreeAsync(dev, s));
   return B200SHM_OK;
 }
 
@@ -407,15 +637,11 @@ int alltoall_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
   Members m = members(pe_start, pe_stride, P);
   const char *sp = m.first + src_off;
   char *dp = m.first + dest_off;
-  const uint64_t pairs = (uint64_t)P * P;
-  const uint64_t bits = src_off | dest_off | B | m.step;
-  const uint64_t w = bits & 15 ? (bits & 7 ? (bits & 3 ? 1 : 4) : 8) : 16;
-  if (B / w < kFlatWords) {
-    /* small blocks: threads over the flattened [pair][word] space */
-    const uint64_t nw = B / w;
-    const unsigned g = grid_for(pairs * nw, 256, 8);
+  const uint64_t bits = src_off | dest_off | B;
+  if (B < 16) { /* more than two blocks may meet in a vector */
+    const uint64_t w = bits & 7 ? (bits & 3 ? 1 : 4) : 8, nw = B / w;
+    const unsigned g = grid_for((uint64_t)P * P * nw, 256, 8);
     switch (w) {
-    case 16: k_alltoall_flat<uint4><<<g, 256, 0, s>>>(sp, dp, m.step, P, nw); break;
     case 8: k_alltoall_flat<unsigned long long><<<g, 256, 0, s>>>(sp, dp, m.step, P, nw); break;
     case 4: k_alltoall_flat<unsigned><<<g, 256, 0, s>>>(sp, dp, m.step, P, nw); break;
     default: k_alltoall_flat<unsigned char><<<g, 256, 0, s>>>(sp, dp, m.step, P, nw); break;
@@ -423,14 +649,32 @@ int alltoall_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
     count_launch();
     return B200SHM_OK;
   }
-  const bool vec = w == 16;
-  const uint64_t n = vec ? B / 16 : B;
-  const unsigned gy = (unsigned)(pairs < kMaxGridY ? pairs : kMaxGridY);
-  dim3 grid(x_blocks(vec ? (n + 3) / 4 : n, gy, 8ull * st().sm_count * 4), gy);
-  if (vec)
-    k_alltoall<true><<<grid, 256, 0, s>>>(sp, dp, m.step, P, B);
-  else
-    k_alltoall<false><<<grid, 256, 0, s>>>(sp, dp, m.step, P, B);
+  const uint64_t nv = (((uintptr_t)dp & 15) + (uint64_t)P * B + 15) / 16; /* vectors of a row */
+  const unsigned gy = (unsigned)((uint64_t)P < kMaxGridY ? (uint64_t)P : kMaxGridY);
+  auto grid = [&](int u) { return dim3((unsigned)((nv + 256 * u - 1) / (256 * u)), gy); };
+  /* More vectors a thread once the grid fills the SMs four times over (below
+   * that the fewer CTAs cost more than the loads in flight give).  Shifted
+   * blocks: a warp in whose bytes a block ends takes about three times as
+   * long, so small blocks want short runs.  128 members, U = 1 / 2 / 4:
+   * 1004 bytes 12.4 / 12.4 us, 2052 18.6 / 16.5, 4100 37.0 / 29.1 / 35.0,
+   * 9999 82 / 59.5 / 68, 16388 - / 90.5 / 96.3, 24580 - / 131 / 133,
+   * 65532 (four) 321. */
+  const bool many = nv * (uint64_t)P >= 16ull * 256 * st().sm_count;
+  /* blocks no larger than a CTA's bytes divide by a reciprocal */
+  auto recip = [&](uint64_t u) { return B <= 4096 * u ? (unsigned)((1ull << 32) / B) + 1 : 0u; };
+  if ((bits & 15) == 0) {
+    if (many)
+      k_alltoall<4><<<grid(4), 256, 0, s>>>(sp, dp, m.step, P, B, recip(4));
+    else
+      k_alltoall<1><<<grid(1), 256, 0, s>>>(sp, dp, m.step, P, B, recip(1));
+  } else {
+    if (many && B >= 32768)
+      k_alltoall_shift<4><<<grid(4), 256, 0, s>>>(sp, dp, m.step, P, B, recip(4));
+    else if (many && B >= 2048)
+      k_alltoall_shift<2><<<grid(2), 256, 0, s>>>(sp, dp, m.step, P, B, recip(2));
+    else
+      k_alltoall_shift<1><<<grid(1), 256, 0, s>>>(sp, dp, m.step, P, B, recip(1));
+  }
   count_launch();
   return B200SHM_OK;
 }
@@ -504,14 +748,8 @@ int broadcast_launch(int root, int pe_start, int pe_stride, int P, uint64_t dest
     return fail(B200SHM_ERR_ARG, "broadcast: dest and source overlap");
   if (nbytes == 0 || P == 1) return B200SHM_OK;
   Members m = members(pe_start, pe_stride, P);
-  const bool vec = ((src_off | dest_off | nbytes | m.step) & 15u) == 0;
-  const uint64_t n = vec ? nbytes / 16 : nbytes;
-  const char *src = m.first + (uint64_t)root * m.step + src_off;
-  if (vec)
-    k_broadcast<true><<<grid_for(n, 256, 8), 256, 0, s>>>(src, m.first + dest_off, m.step, P, root, nbytes);
-  else
-    k_broadcast<false><<<grid_for(n, 256, 8), 256, 0, s>>>(src, m.first + dest_off, m.step, P, root, nbytes);
-  count_launch();
+  spread(m.first + (uint64_t)root * m.step + src_off, m.first + dest_off, m.step, P, nbytes, 1,
+         root, Even{nbytes}, s);
   return B200SHM_OK;
 }
 
