@@ -15,10 +15,11 @@
  *    word;
  *  - every request is cut into tiles on the host (a range of elements of a
  *    reduction, a chunk or a run of segments of a copy, one atomic) and
- *    its tiles into at most one share per CTA; a CTA claims a share with
- *    one fetch-and-add on the slot's claim word, only on requests already
- *    mirrored, so no CTA ever holds a claim it cannot serve and no CTA
- *    ever waits for another CTA;
+ *    its tiles into at most one share per CTA; a CTA looks over the claim
+ *    words of the 32 oldest open requests and claims a share with one
+ *    fetch-and-add on one of them, only on requests already mirrored, so
+ *    no CTA ever holds a claim it cannot serve and no CTA ever waits for
+ *    another CTA;
  *  - the CTA that finishes a request's last tile writes its completion word
  *    (sequence, AMO old value, status) to host memory after a system-scope
  *    fence;
@@ -176,7 +177,7 @@ static_assert(offsetof(SCtl, down) == 64 && sizeof(SCtl) == 128, "host and devic
 
 /* Device-side state. */
 struct SDev {
-  unsigned long long cursor;      /* the request whose tiles are handed out  */
+  unsigned long long cursor;      /* no request below it has shares left      */
   unsigned long long tail_mirror; /* last tail a CTA read from host memory   */
   unsigned int poll_lock;         /* one CTA at a time reads host memory     */
   int stop;                       /* the host's stop flag, as last read      */
@@ -224,23 +225,18 @@ __device__ __forceinline__ unsigned long long now_ns() {
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ void copy_words(SReq *dst, const SReq *src) {
-  const volatile unsigned long long *s = (const volatile unsigned long long *)src;
-  unsigned long long *d = (unsigned long long *)dst;
-#pragma unroll
-  for (int i = 0; i < 16; i++) d[i] = s[i];
-}
-
 /* The device mirror of the ring: the CTA that holds the poll lock copies
  * newly published requests from host memory into it (sequence word last)
  * before it opens them to claims, so the other CTAs read requests from L2
- * only.  Copy request r into *out, for a CTA that holds a share of r (the
- * caller has fenced after its claim): the slot keeps r until r completes,
- * which needs that share, so one copy is consistent; 1 when the copy is of
- * r (always, by that argument). */
-__device__ int copy_req(const SArgs &a, unsigned long long r, SReq *out) {
-  copy_words(out, &a.mreq[r % a.Q]);
-  return out->seq == r + 1 ? 1 : 0;
+ * only.  Copy request r into *out (shared memory), a word per lane, for a
+ * CTA that holds a share of r (its warp has fenced after the claim): the
+ * slot keeps r until r completes, which needs that share, so one copy is
+ * consistent; true when the copy is of r (always, by that argument). */
+__device__ bool copy_req(const SArgs &a, unsigned long long r, SReq *out, int lane) {
+  if (lane < 16)
+    ((unsigned long long *)out)[lane] = vld((const unsigned long long *)&a.mreq[r % a.Q] + lane);
+  __syncwarp();
+  return out->seq == r + 1;
 }
 
 /* Requests one poll copies at most (B200SHM_SERVE_MIRROR_BATCH overrides
@@ -250,83 +246,130 @@ __device__ int copy_req(const SArgs &a, unsigned long long r, SReq *out) {
  * fetch-adds/s), 64 served 1.08 M (1.93 M), 256 served 1.16 M (2.29 M). */
 constexpr unsigned kMirrorBatch = 256;
 
-/* Claim the next tiles (thread 0).  Returns 1 with request *cr, tiles
- * [*ct, *ct + *count) and the request in *req; 2 when this CTA took the poll
- * lock and found requests [*mfrom, *mupto) published but not yet copied
- * into device memory (the CTA copies them, then publishes and releases the
- * lock); or 0 when the CTA should exit (stop requested or idle past the
- * limit, in both cases holding no claim).
- * A claim is one fetch-and-add of 1 on the slot's claim word, which says
- * by itself whether a share was left: no request descriptor is read before
- * the claim, and a CTA that finds nothing left walks on to the next
- * request at once (the cursor is only a hint of where unclaimed shares
- * start; whoever takes a request's last share moves it on).  An add that
+/* Claim the next tiles (the CTA's first warp).  Returns 1 with request *cr,
+ * tiles [*ct, *ct + *count) and the request in *req; 2 when this CTA took
+ * the poll lock and found requests [*mfrom, *mupto) published but not yet
+ * copied into device memory (the CTA copies them, then publishes and
+ * releases the lock); or 0 when the CTA should exit (stop requested or idle
+ * past the limit, in both cases holding no claim).
+ * The warp reads the claim words of the 32 oldest requests that may have
+ * shares left, counts the shares left in them, and takes one by a fetch-
+ * and-add of 1 on the claim word of the request that holds the
+ * (blockIdx.x mod shares left)-th: CTAs that look at the same moment aim
+ * at different shares.  The word says by itself whether the share was
+ * left.  (A CTA that tried the requests one after the other, all CTAs the
+ * same ones, spent an atomic's round trip on each request whoever served
+ * it: 2048 fetch-adds took 905 us, 413 now, which the host's turns take;
+ * a request every 5 us sees 18 us either way.)  An add that
  * lands after the slot moved on to a later request x (only possible once
  * the request it aimed at is complete) holds a share of x, which is served
- * as such, so no tile is ever lost or handed out twice.  *r_hint carries
- * the request this CTA looks at next from one claim to the next. */
+ * as such, so no tile is ever lost or handed out twice.  The cursor is
+ * where unclaimed shares start, and *r_hint this CTA's copy of it: a scan
+ * moves them past the requests at its start that have none left. */
 __device__ int claim(const SArgs &a, SReq *req, unsigned long long *cr, unsigned long long *ct,
                      unsigned *count, unsigned long long *mfrom, unsigned long long *mupto,
-                     unsigned long long idle_since, unsigned long long *r_hint) {
+                     unsigned long long idle_since, unsigned long long *r_hint, int lane) {
   unsigned backoff = 32;
   unsigned long long r = *r_hint;
   for (;;) {
-    const unsigned long long cur = vld(&a.dev->cursor);
-    const unsigned long long tl = vld(&a.dev->tail_mirror);
+    unsigned long long cur = 0, tl = 0;
+    if (lane == 0) {
+      cur = vld(&a.dev->cursor);
+      tl = vld(&a.dev->tail_mirror);
+    }
+    cur = __shfl_sync(~0u, cur, 0);
+    tl = __shfl_sync(~0u, tl, 0);
     if (cur > r) r = cur;
     if (r >= tl) {
-      /* test, then test-and-set: waiting CTAs only read the lock word */
-      if (*(const volatile unsigned *)&a.dev->poll_lock == 0u &&
-          atomicCAS(&a.dev->poll_lock, 0u, 1u) == 0u) {
-        const unsigned long long mt = vld(&a.dev->tail_mirror);
-        const unsigned long long hv = ld_acquire_sys(&a.ctl->tail);
-        const unsigned long long ht = hv & ~kStopBit;
-        /* a stop takes effect once every published request is in the
-         * mirror (with a heap budget some may still wait for room), so the
-         * loop drains before it exits */
-        if ((hv & kStopBit) && ht == mt) *(volatile int *)&a.dev->stop = 1;
-        if (ht > mt) { /* the whole CTA copies them, still holding the lock */
-          *mfrom = mt;
-          *mupto = ht < mt + a.mirror_batch ? ht : mt + a.mirror_batch;
-          *r_hint = r;
-          return 2;
+      int go = -1;
+      if (lane == 0) {
+        /* test, then test-and-set: waiting CTAs only read the lock word */
+        if (*(const volatile unsigned *)&a.dev->poll_lock == 0u &&
+            atomicCAS(&a.dev->poll_lock, 0u, 1u) == 0u) {
+          const unsigned long long mt = vld(&a.dev->tail_mirror);
+          const unsigned long long hv = ld_acquire_sys(&a.ctl->tail);
+          const unsigned long long ht = hv & ~kStopBit;
+          /* a stop takes effect once every published request is in the
+           * mirror (with a heap budget some may still wait for room), so the
+           * loop drains before it exits */
+          if ((hv & kStopBit) && ht == mt) *(volatile int *)&a.dev->stop = 1;
+          if (ht > mt) { /* the whole CTA copies them, still holding the lock */
+            *mfrom = mt;
+            *mupto = ht < mt + a.mirror_batch ? ht : mt + a.mirror_batch;
+            go = 2;
+          } else {
+            atomicExch(&a.dev->poll_lock, 0u);
+          }
         }
-        atomicExch(&a.dev->poll_lock, 0u);
+        if (go < 0 && vld(&a.dev->tail_mirror) <= r) {
+          /* only the lock holder reads host memory: a read of host memory by
+           * every waiting CTA on every turn floods the path to the host and
+           * stalls every other memory access behind it */
+          if (*(const volatile int *)&a.dev->stop) {
+            go = 0;
+          } else {
+            /* idle is the loop's idle time, not this CTA's: a CTA that wins no
+             * claim for a while stays as long as requests keep arriving */
+            const unsigned long long act = vld(&a.dev->last_active), now = now_ns();
+            const unsigned long long since = act > idle_since ? act : idle_since;
+            if (now > since && now - since > a.idle_ns) {
+              go = 0;
+            } else {
+              __nanosleep(backoff);
+              backoff = backoff < 128 ? backoff * 2 : 128;
+            }
+          }
+        }
       }
-      if (vld(&a.dev->tail_mirror) <= r) {
-        /* only the lock holder reads host memory: a read of host memory by
-         * every waiting CTA on every turn floods the path to the host and
-         * stalls every other memory access behind it */
-        if (*(const volatile int *)&a.dev->stop) return 0;
-        /* idle is the loop's idle time, not this CTA's: a CTA that wins no
-         * claim for a while stays as long as requests keep arriving */
-        const unsigned long long act = vld(&a.dev->last_active), now = now_ns();
-        const unsigned long long since = act > idle_since ? act : idle_since;
-        if (now > since && now - since > a.idle_ns) return 0;
-        __nanosleep(backoff);
-        backoff = backoff < 128 ? backoff * 2 : 128;
+      go = __shfl_sync(~0u, go, 0);
+      if (go >= 0) {
+        *r_hint = r;
+        return go;
       }
       continue;
     }
     fence_gpu(); /* the claim words of requests below tail_mirror are set */
-    for (; r < tl; r++) {
-      const unsigned long long old = atomicAdd(&a.tctr[r % a.Q], 1ull);
-      const unsigned long long x = r + (((old >> kTagShift) - r) & kField24);
-      const unsigned long long nsh = (old >> kShareShift) & 0xFFFFull, sh = old & kField24;
-      /* r is handed out: the cursor moves past it (a CTA that finds the
-       * shares gone leaves that to the one that took the last) */
-      if (x != r || sh + 1 == nsh) atomicMax(&a.dev->cursor, r + 1);
-      if (sh >= nsh) continue;
-      /* share sh of request x is ours; x stays in its slot until it completes */
-      fence_gpu();
-      if (req->seq != x + 1 && !copy_req(a, x, req)) continue; /* not reached */
+    __syncwarp();
+    const unsigned long long mine = r + lane;
+    unsigned left = 0; /* shares left in request r + lane */
+    if (mine < tl) {
+      const unsigned long long w = vld(&a.tctr[mine % a.Q]);
+      const unsigned nsh = (unsigned)(w >> kShareShift) & 0xFFFFu;
+      const unsigned long long sh = w & kField24;
+      if ((w >> kTagShift) == (mine & kField24) && sh < nsh) left = nsh - (unsigned)sh;
+    }
+    const unsigned open = __ballot_sync(~0u, left != 0);
+    /* the requests before the first open one are handed out */
+    r = open ? r + (unsigned)(__ffs(open) - 1) : r + 32 < tl ? r + 32 : tl;
+    if (lane == 0 && r > cur) atomicMax(&a.dev->cursor, r);
+    if (!open) continue;
+    unsigned upto = left; /* shares left in the requests up to this lane's */
+#pragma unroll
+    for (int d = 1; d < 32; d *= 2) {
+      const unsigned o = __shfl_up_sync(~0u, upto, d);
+      if (lane >= d) upto += o;
+    }
+    const unsigned pick = blockIdx.x % __shfl_sync(~0u, upto, 31);
+    const int from = __ffs(__ballot_sync(~0u, pick < upto)) - 1;
+    const unsigned long long aim = __shfl_sync(~0u, mine, from);
+    unsigned long long old = 0;
+    if (lane == 0) old = atomicAdd(&a.tctr[aim % a.Q], 1ull);
+    old = __shfl_sync(~0u, old, 0);
+    const unsigned long long x = aim + (((old >> kTagShift) - aim) & kField24);
+    const unsigned long long nsh = (old >> kShareShift) & 0xFFFFull, sh = old & kField24;
+    if (sh >= nsh) continue; /* another CTA was first: look again */
+    /* share sh of request x is ours; x stays in its slot until it completes */
+    fence_gpu();
+    __syncwarp();
+    if (!copy_req(a, x, req, lane)) continue; /* not reached */
+    if (lane == 0) {
       const unsigned long long k = share_tiles(req->ntiles, gridDim.x);
       *cr = x;
       *ct = sh * k;
       *count = (unsigned)(req->ntiles - sh * k < k ? req->ntiles - sh * k : k);
-      *r_hint = x == r && sh + 1 < nsh ? r : r + 1;
-      return 1;
     }
+    *r_hint = r;
+    return 1;
   }
 }
 
@@ -711,13 +754,16 @@ __global__ void __launch_bounds__(kServeThreads) k_serve(const SArgs a) {
   __shared__ unsigned long long s_tclaim;
   unsigned long long idle_since = now_ns();
   unsigned long long r_hint = 0;
-  if (threadIdx.x == 0) s_req.seq = 0;
   for (;;) {
-    if (threadIdx.x == 0) {
-      s_go = claim(a, &s_req, &s_cr, &s_ct, &s_count, &s_mfrom, &s_mupto, idle_since, &r_hint);
-      s_tclaim = now_ns();
-      s_fetched = 0;
-      s_status = 0;
+    if (threadIdx.x < 32) {
+      const int go = claim(a, &s_req, &s_cr, &s_ct, &s_count, &s_mfrom, &s_mupto, idle_since,
+                           &r_hint, (int)threadIdx.x);
+      if (threadIdx.x == 0) {
+        s_go = go;
+        s_tclaim = now_ns();
+        s_fetched = 0;
+        s_status = 0;
+      }
     }
     __syncthreads();
     if (!s_go) {
