@@ -1250,13 +1250,19 @@ int b200shm_serve_replay(b200shm_server *s, const b200shm_request *reqs, uint64_
     return B200SHM_OK;
   }
   std::vector<uint64_t> tickets(n);
+  std::vector<char> taken(n, 0); /* the completion has been read */
   std::vector<uint64_t> pend;
   pend.reserve(s->Q);
-  uint64_t k = 0, done = 0;
+  uint64_t k = 0, done = 0, oldest = 0; /* requests below `oldest` are taken */
   double last_progress = host_now();
   for (unsigned it = 0; done < n; it++) {
     const double now = host_now();
-    if (k < n && now - t0 >= arrival_s[k]) {
+    /* A slot may be reused as soon as its request is complete, so a request
+     * waits until the completion that its slot holds has been read: else the
+     * loop, when it is as fast as this thread, overwrites it. */
+    while (oldest < k && taken[oldest]) oldest++;
+    if (k < n && now - t0 >= arrival_s[k] &&
+        (oldest == k || s->tail - tickets[oldest] < s->Q)) {
       uint64_t tk;
       const int rc = b200shm_serve_enqueue(s, &reqs[k], &tk);
       if (rc == B200SHM_OK) {
@@ -1276,6 +1282,7 @@ int b200shm_serve_replay(b200shm_server *s, const b200shm_request *reqs, uint64_
       if (rc == 1) {
         latency_s[j] = host_now() - t0 - arrival_s[j];
         if (fetched) fetched[j] = f;
+        taken[j] = 1;
         pend[i] = pend.back();
         pend.pop_back();
         done++;
