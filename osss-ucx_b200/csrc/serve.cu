@@ -265,12 +265,17 @@ constexpr unsigned kMirrorBatch = 256;
  * the request it aimed at is complete) holds a share of x, which is served
  * as such, so no tile is ever lost or handed out twice.  The cursor is
  * where unclaimed shares start, and *r_hint this CTA's copy of it: a scan
- * moves them past the requests at its start that have none left. */
+ * moves them past the requests at its start that have none left.
+ * Block 0 looks for published requests before each claim, so that they are
+ * copied while the others serve the batch before (2048 all-to-alls of 4
+ * members x 64 KiB: 1727 -> 1595 us); with a heap budget it waits for the
+ * batch to be handed out, as the others do. */
 __device__ int claim(const SArgs &a, SReq *req, unsigned long long *cr, unsigned long long *ct,
                      unsigned *count, unsigned long long *mfrom, unsigned long long *mupto,
                      unsigned long long idle_since, unsigned long long *r_hint, int lane) {
   unsigned backoff = 32;
   unsigned long long r = *r_hint;
+  bool look_first = blockIdx.x == 0 && gridDim.x > 1 && !a.budget;
   for (;;) {
     unsigned long long cur = 0, tl = 0;
     if (lane == 0) {
@@ -280,7 +285,8 @@ __device__ int claim(const SArgs &a, SReq *req, unsigned long long *cr, unsigned
     cur = __shfl_sync(~0u, cur, 0);
     tl = __shfl_sync(~0u, tl, 0);
     if (cur > r) r = cur;
-    if (r >= tl) {
+    if (r >= tl || look_first) {
+      look_first = false;
       int go = -1;
       if (lane == 0) {
         /* test, then test-and-set: waiting CTAs only read the lock word */
@@ -326,7 +332,7 @@ __device__ int claim(const SArgs &a, SReq *req, unsigned long long *cr, unsigned
         *r_hint = r;
         return go;
       }
-      continue;
+      if (r >= tl) continue;
     }
     fence_gpu(); /* the claim words of requests below tail_mirror are set */
     __syncwarp();
