@@ -237,7 +237,7 @@ struct Lane {
 
 /* One column group's work on the column whose first element is e0 (live:
  * the column exists; the whole warp enters, for the shuffles).  C: leaves a
- * lane of a tree holds -- 2, 4, 8: all loaded at once; 16, 32: chunks of 8;
+ * lane of a tree holds -- 2, 4, 8: all loaded at once; 16 to 128: chunks of 8;
  * 0: any number of chunks of 8, a binary counter over them; kRagged<L>:
  * fewer than 2^L leaves, not a power of two (a binomial tree in one lane):
  * chunks of 8, then the last leaves one by one.
@@ -327,25 +327,36 @@ __device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, ui
       typedef std::integral_constant<int, 8> k8;
       if constexpr (C >= 2 && C <= 8) {
         r = chunk(l0, std::integral_constant<int, C>{});
-      } else if constexpr (C == 16) {
-        /* two chunks, one at a time (keeps 8 loads in flight, not 16) */
+      } else if constexpr (C >= 16) {
+        /* C / 8 chunks, one at a time (8 loads in flight, not C), each
+         * combined with the finished subtrees of its size before it: a
+         * binary counter whose carries are branches all lanes take alike */
+        PK s0, s1, s2, s3;
 #pragma unroll 1
-        for (int c2 = 0; c2 < 2; c2++) {
-          const PK y = chunk(l0 + 8 * c2, k8{});
-          r = c2 ? comb(r, y) : y;
-        }
-      } else if constexpr (C == 32) {
-        /* four chunks, one at a time: ((c0 c1)(c2 c3)) with two slots */
-        PK h, s2;
-#pragma unroll 1
-        for (int c4 = 0; c4 < 4; c4++) {
-          PK y = chunk(l0 + 8 * c4, k8{});
-          if (c4 & 1) {
-            y = comb(h, y);
-            if (c4 == 1) s2 = y;
-            else r = comb(s2, y);
+        for (int c8 = 0; c8 < C / 8; c8++) {
+          r = chunk(l0 + 8 * c8, k8{});
+          if (c8 & 1) {
+            r = comb(s0, r);
+            if constexpr (C >= 32) {
+              if (c8 & 2) {
+                r = comb(s1, r);
+                if constexpr (C >= 64) {
+                  if (c8 & 4) {
+                    r = comb(s2, r);
+                    if constexpr (C >= 128) {
+                      if (c8 & 8) r = comb(s3, r);
+                      else s3 = r;
+                    }
+                  } else {
+                    s2 = r;
+                  }
+                }
+              } else {
+                s1 = r;
+              }
+            }
           } else {
-            h = y;
+            s0 = r;
           }
         }
       } else {
@@ -466,7 +477,7 @@ constexpr int min_ctas() {
   if (MODE == kBytes) return 1;
   if (MM) return 3;
   if (ORDER == ORD_CHAIN) return sizeof(T) < 4 ? 2 : sizeof(T) == 4 || EDGES ? 4 : 5;
-  return C == 0 || C < -3 ? 2 : !POW2 ? 3 : EDGES ? 4 : 5;
+  return C == 0 || C < -3 ? 2 : !POW2 ? 3 : EDGES || C > 32 ? 4 : 5;
 }
 template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2, int MODE, bool EDGES>
 __global__ void __launch_bounds__(256, min_ctas<T, ORDER, MM, C, POW2, MODE, EDGES>())
@@ -569,24 +580,37 @@ void launch_edges(uint64_t lanes, cudaStream_t s, const RArgs &a) {
   launch_one(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, false>, lanes, s, a);
 }
 
+/* Whether a lane has instances of 64 and 128 leaves (not long double, whose
+ * software arithmetic bounds it, and takes minutes to compile). */
+template <class T, int MODE>
+constexpr bool kLongRuns = MODE == kPacks && !std::is_same<T, f80>::value;
 /* leaves per lane n -> the instance */
 template <class T, int OP, int ORDER, int V, bool POW2, int MODE>
 void launch_tree(int n, uint64_t lanes, cudaStream_t s, const RArgs &a) {
   constexpr int C16 = MODE == kPacks ? 16 : 0, C32 = MODE == kPacks ? 32 : 0;
+  constexpr int C64 = kLongRuns<T, MODE> ? 64 : 0, C128 = kLongRuns<T, MODE> ? 128 : 0;
   switch (n) {
   case 2: launch_edges<T, OP, ORDER, V, false, 2, POW2, MODE>(lanes, s, a); break;
   case 4: launch_edges<T, OP, ORDER, V, false, 4, POW2, MODE>(lanes, s, a); break;
   case 8: launch_edges<T, OP, ORDER, V, false, 8, POW2, MODE>(lanes, s, a); break;
   case 16: launch_edges<T, OP, ORDER, V, false, C16, POW2, MODE>(lanes, s, a); break;
   case 32: launch_edges<T, OP, ORDER, V, false, C32, POW2, MODE>(lanes, s, a); break;
+  case 64: launch_edges<T, OP, ORDER, V, false, C64, POW2, MODE>(lanes, s, a); break;
+  case 128: launch_edges<T, OP, ORDER, V, false, C128, POW2, MODE>(lanes, s, a); break;
   default: launch_edges<T, OP, ORDER, V, false, 0, POW2, MODE>(lanes, s, a); break;
   }
 }
 
 /* Lanes per column (log2), for `cols` columns over `leaves` leaves.
  * Many columns: 2 lanes (1 where a lane would hold fewer than 8 leaves); for
- * float trees as many as give each lane 32 leaves (2 to 8).  On the 64-PE
- * workload G = 2 with 32 leaves per lane ran the f32 tree at 5.6-5.9 TB/s,
+ * float trees as many as give each lane `run` leaves (2 to 8): 128, the
+ * most an instance without a stack takes, from 256 leaves on, and from 128
+ * where every member is a leaf and every column a pack; else 32.  (f32 SUM,
+ * 200 MiB: 256 members at 8 lanes of 32, a warp reading 64 bytes of each
+ * member, 2.82 TB/s, at 2 of 128 5.50; 128 members at 4 of 32 4.89, at 2 of
+ * 64 5.70; but 128 to 255 members with extras or edges at 2 lanes 1-8 %
+ * slower.)  Long runs only where at least 256 threads an SM are left: 256
+ * members x 65536 at 4 of 64 4.36 TB/s, at 8 of 32 2.6.  On the 64-PE workload G = 2 with 32 leaves per lane ran the f32 tree at 5.6-5.9 TB/s,
  * G = 4 with 16 at 5.2-5.4 (a warp then reads 128 rather than 256
  * consecutive bytes of each member per load).  Few columns: what counts is
  * how many rounds of loads a lane makes in turn, so lanes are added while a
@@ -599,13 +623,15 @@ void launch_tree(int n, uint64_t lanes, cudaStream_t s, const RArgs &a) {
  * B200SHM_REDUCE_COOP sets the starting point (0 or 1 = one lane per
  * column). */
 template <int ORDER>
-int lanes_log2(uint64_t cols, int leaves, bool wide) {
+int lanes_log2(uint64_t cols, int leaves, bool wide, int run) {
   int G = wide ? 1 : 2; /* 16-byte elements: a chain of one lane per element */
-  if (ORDER != ORD_CHAIN) G = std::max(2, std::min(8, leaves / 32));
+  if (ORDER != ORD_CHAIN) G = std::max(2, std::min(8, leaves / run));
   static const char *ec = getenv("B200SHM_REDUCE_COOP"); /* read once */
   if (ec) G = std::max(1, std::min(8, atoi(ec)));
   int lg = 31 - __builtin_clz((unsigned)G);
   while (lg > 0 && (8 << lg) > leaves) lg--;
+  if (!ec && ORDER != ORD_CHAIN) /* long runs only where they fill the SMs */
+    while (lg < 3 && (leaves >> lg) > 32 && (cols << lg) < (uint64_t)grid_sms() * 256) lg++;
   if (!ec)
     while (lg < 4 && (4 << (lg + 1)) <= leaves &&
            (cols << (2 * lg)) < (uint64_t)grid_sms() * 128)
@@ -624,7 +650,9 @@ void run_mode(RArgs &a, cudaStream_t s) {
    * butterflies, and for binomial trees over power-of-two teams */
   constexpr bool any_order = ORDER == ORD_CHAIN && (std::is_integral<T>::value || MM);
   const bool split = any_order || ORDER == ORD_BUTTERFLY || (ORDER == ORD_BINOMIAL && pow2);
-  a.lgG = split ? lanes_log2<ORDER>(a.nvec + a.nedge, leaves, sizeof(T) == 16) : 0;
+  const bool long_runs = kLongRuns<T, MODE> && (leaves >= 256 || (pow2 && a.nedge == 0));
+  const int run = long_runs ? 128 : 32;
+  a.lgG = split ? lanes_log2<ORDER>(a.nvec + a.nedge, leaves, sizeof(T) == 16, run) : 0;
   const uint64_t lanes = std::max<uint64_t>(a.nvec + a.nedge, 1) << a.lgG;
   if constexpr (ORDER == ORD_CHAIN) {
     launch_edges<T, OP, ORDER, V, MM, 1, true, MODE>(lanes, s, a);
