@@ -685,7 +685,7 @@ def run_movement(args, world, rank, local):
         "alltoalls64": (lambda: B.alltoalls(as_d, as_s, 2, 3, NS, 8, team=team, stream=s_ptr),
                         2 * PM * PM * NS * 8, "GB/s", "k_alltoalls"),
         "fcollect64": (lambda: B.fcollect(fc_d, fc_s, NF * 8, team=team, stream=s_ptr),
-                       PM * NF * 8 + PM * PM * NF * 8, "GB/s", "k_fcollect"),
+                       PM * NF * 8 + PM * PM * NF * 8, "GB/s", "k_spread"),
         "atomic_fetch_add": (lambda: B.amo_batch("fetch_add", "int64", NOPS, d["pe"], d["off"],
                                                  d["val"], None, d["f"], stream=s_ptr),
                              NOPS, "Mops/s", "k_amo"),
