@@ -3,11 +3,17 @@ against each other, blocks below, at and around a vector and a CTA's tile,
 empty contributions, blocks whose ends meet inside one vector; per call and
 through the serving loop.  Byte for byte against the oracle (or the rows'
 concatenation); bytes beside the dest stay untouched."""
+import os
+import subprocess
+import sys
+import textwrap
+
 import numpy as np
 import pytest
 
 import gen
 
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 pytestmark = pytest.mark.gpu
 GUARD = 64
 SHIFTS = [(0, 0), (1, 0), (0, 5), (4, 12), (8, 0), (15, 15), (3, 14)]
@@ -98,3 +104,36 @@ def test_served_copies_shifted(B, heap, rs, nb):
                         assert (got[j] == exp).all(), (kind, a, b, j)
     finally:
         srv.stop()
+
+
+WIDE_COLLECT = textwrap.dedent("""
+    import sys
+    import numpy as np
+    sys.path[:0] = [{pkg!r}]
+    import b200shm as B
+    B.init(1100, 1 << 20)
+    rng = np.random.default_rng(3)
+    for P, most in ((135, 50), (136, 50), (1031, 40), (1032, 40), (1100, 3)):
+        team, counts = (0, 1, P), rng.integers(0, most + 1, P)
+        x = rng.integers(0, 256, (P, most), dtype=np.uint8)
+        want = np.concatenate([x[k, :c] for k, c in enumerate(counts)])
+        for a, b in ((0, 0), (3, 5)):
+            src, dst = B.malloc(most + 16), B.malloc(len(want) + 32)
+            B.put_rows(src + a, x, team=team)
+            B.memset(dst, 0xA5, len(want) + 32, team=team)
+            B.collect(dst + b, src + a, counts.astype(np.uint64), team=team)
+            got = B.get_rows(dst, len(want) + 32, np.uint8, team=team)
+            assert (got[:, b:b + len(want)] == want).all(), (P, a, b)
+            assert (got[:, :b] == 0xA5).all() and (got[:, b + len(want):] == 0xA5).all()
+            B.free(src); B.free(dst)
+    B.finalize()
+    print("ok")
+""")
+
+
+def test_collect_of_wide_teams():
+    """Size tables of each kind: the small and the large kernel parameter, and
+    the one in device memory, on both sides of their limits."""
+    code = WIDE_COLLECT.format(pkg=os.path.join(ROOT, "osss-ucx_b200"))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip().endswith("ok"), r.stdout + r.stderr
