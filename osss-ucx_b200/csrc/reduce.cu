@@ -36,7 +36,7 @@ static int reduce_check(int op, int dtype, int algo, int pe_size) {
     return fail(B200SHM_ERR_UNSUPPORTED, "reduce: op %d is not defined on dtype %d", op, dtype);
   if (pe_size < 1) return fail(B200SHM_ERR_ARG, "reduce: team size %d < 1", pe_size);
   int p2s = 1;
-  while (p2s * 2 <= pe_size) p2s *= 2;
+  while (p2s <= pe_size / 2) p2s *= 2;
   const bool tree = !is_int && op != B200SHM_MIN && op != B200SHM_MAX && algo != B200SHM_LINEAR;
   const int leaves = algo == B200SHM_BINOMIAL ? pe_size : p2s;
   if (tree && leaves > (1 << (kMaxLevels - 1)))
@@ -56,7 +56,7 @@ static RArgs reduce_args(const char *src, char *dst, uint64_t sstep, uint64_t ds
                          uint64_t nelems, int algo) {
   RArgs a;
   int logp = 0, p2s = 1;
-  while (p2s * 2 <= P) {
+  while (p2s <= P / 2) {
     p2s *= 2;
     logp++;
   }

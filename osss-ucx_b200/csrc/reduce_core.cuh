@@ -444,6 +444,13 @@ __device__ __forceinline__ bool p2s_extra(int q, int P, int p2s) {
   return (long long)(as + 1) * p2s / P == q;
 }
 
+/* The first of lane g's leaves where 2^lgG lanes share n: lane g has
+ * [lane_leaf(g), lane_leaf(g + 1)).  64-bit products: integer and linear
+ * reductions over buffers of the caller's have up to 2^31 - 1 members. */
+__host__ __device__ __forceinline__ int lane_leaf(int g, int n, int lgG) {
+  return (int)(((unsigned long long)g * (unsigned)n) >> lgG);
+}
+
 constexpr int kMaxLevels = 13; /* trees of up to 4096 leaves */
 
 /* ---- exact replay for order-dependent MIN/MAX elements ----------------- */

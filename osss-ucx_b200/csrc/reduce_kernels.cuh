@@ -266,24 +266,25 @@ __device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, ui
     if constexpr (ORDER == ORD_CHAIN) {
       const char *p = src + (uint64_t)l0 * a.sstep;
       r = ld_col<T, V, MODE>(p);
-      int j = l0 + 1;
+      unsigned j = (unsigned)l0 + 1; /* l1 may be the largest int: j + 8 is above it */
+      const unsigned end = (unsigned)l1;
       do { /* once at least: a MIN/MAX lane looks at its first operand below the loads */
         PK x[8];
         const uint64_t step = opaque(a.sstep);
 #pragma unroll
         for (int u = 0; u < 8; u++)
-          if (j + u < l1) x[u] = ld_col<T, V, MODE>(p + (uint64_t)(u + 1) * step);
+          if (j + u < end) x[u] = ld_col<T, V, MODE>(p + (uint64_t)(u + 1) * step);
         p += 8 * step;
         if constexpr (MM)
-          if (j == l0 + 1) cls = mm_flags<OP>(r);
+          if (j == (unsigned)l0 + 1) cls = mm_flags<OP>(r);
 #pragma unroll
         for (int u = 0; u < 8; u++)
-          if (j + u < l1) {
+          if (j + u < end) {
             r = comb(r, x[u]);
             if constexpr (MM) cls |= mm_flags<OP>(x[u]);
           }
         j += 8;
-      } while (j < l1);
+      } while (j < end);
     } else {
       /* K leaves from q0 as a complete subtree, all loads before any use;
        * extra members folded in first as op(extra, own) (reduce.c:232-241) */
@@ -490,8 +491,8 @@ k_reduce(const __grid_constant__ RArgs a) {
   const int c = lane >> lgG, lgcols = 5 - lgG; /* columns per warp per iteration */
   const int P = a.P;
   const int nleaves = ORDER == ORD_BUTTERFLY ? a.p2s : P;
-  ln.l0 = (ln.g * nleaves) >> lgG; /* at most 2^20 members, 16 lanes */
-  ln.l1 = ((ln.g + 1) * nleaves) >> lgG;
+  ln.l0 = lane_leaf(ln.g, nleaves, lgG);
+  ln.l1 = lane_leaf(ln.g + 1, nleaves, lgG);
   if (ORDER == ORD_BUTTERFLY) {
     ln.m0 = (ln.l0 * P + a.p2s - 1) >> a.logp2s;
     ln.m1 = (ln.l1 * P + a.p2s - 1) >> a.logp2s;
