@@ -1019,6 +1019,8 @@ int b200shm_batch_create(b200shm_reduce_desc *descs, uint64_t n, int flags,
     if (rc)
       return bail(fail(rc, "batch descriptor %llu: %s", (unsigned long long)i,
                        b200shm_last_error()));
+    /* tuning runs the whole batch, separate launches included: not in place */
+    if (x.nelems > 0 && x.dest_off == x.src_off) tune = false;
     const int ds = dslot_of(x.dtype, x.op);
     const bool is_int = x.dtype <= B200SHM_U64;
     const bool mm = x.op == B200SHM_MIN || x.op == B200SHM_MAX;
@@ -1072,7 +1074,6 @@ int b200shm_batch_create(b200shm_reduce_desc *descs, uint64_t n, int flags,
       b.fallback.push_back(x); /* trees deeper than one lane's stack */
       continue;
     }
-    if (x.dest_off == x.src_off) tune = false; /* tuning runs the batch: not in place */
     choose_plan(d);
     set_columns(d);
     x.lanes = d.G;
