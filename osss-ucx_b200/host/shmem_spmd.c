@@ -603,8 +603,7 @@ static pthread_mutex_t g_srv_mu = PTHREAD_MUTEX_INITIALIZER;
 static b200shm_server *g_srv;
 typedef struct {
   uint64_t ticket;
-  void *fetch;
-  int size;
+  int fetches; /* its old value goes to the program */
 } nbi_t;
 /* the outstanding requests of one context */
 typedef struct {
@@ -624,9 +623,28 @@ typedef struct {
 static __thread nbi_list_t t_default; /* SHMEM_CTX_DEFAULT of this PE */
 #define t_nbi_n (t_default.n)
 
+/* A ring slot keeps the old value of the fetch it last held until a later
+ * request completes in it, so whoever is about to queue that request first
+ * takes the value to where the program wants it, whichever PE queued the
+ * fetch.  g_nbi_mu orders the requests queued on the ring (nothing else
+ * queues on it), so the slot of the next one is known. */
+#define NBI_SLOTS 4096
+typedef struct {
+  uint64_t ticket;
+  void *fetch; /* NULL: nothing to take */
+  int size;
+} held_t;
+static pthread_mutex_t g_nbi_mu = PTHREAD_MUTEX_INITIALIZER;
+static held_t g_held[NBI_SLOTS];
+static uint64_t g_next_ticket;
+
 static b200shm_server *job_server(void) {
   pthread_mutex_lock(&g_srv_mu);
-  if (!g_srv && b200shm_serve_start(4096, 0, 0.25, &g_srv) != 0) g_srv = NULL;
+  if (!g_srv) {
+    memset(g_held, 0, sizeof(g_held));
+    g_next_ticket = 0;
+    if (b200shm_serve_start(NBI_SLOTS, 0, 0.25, &g_srv) != 0) g_srv = NULL;
+  }
   b200shm_server *s = g_srv;
   pthread_mutex_unlock(&g_srv_mu);
   return s;
@@ -639,14 +657,35 @@ static void stop_job_server(void) {
   pthread_mutex_unlock(&g_srv_mu);
 }
 
+/* Take the old value a slot holds (under g_nbi_mu); 0 while the fetch is not
+ * complete.  A fetch that failed is left to its own PE's quiet. */
+static int take_held(held_t *h) {
+  uint64_t f = 0;
+  const int rc = b200shm_serve_poll(g_srv, h->ticket, &f);
+  if (rc == 0) return 0;
+  if (rc > 0) memcpy(h->fetch, &f, (size_t)h->size);
+  h->fetch = NULL;
+  return 1;
+}
+
+/* Complete one outstanding request. */
+static int nbi_complete(const nbi_t *q) {
+  const int rc = b200shm_serve_wait(g_srv, q->ticket, 60.0, NULL);
+  if (q->fetches) {
+    pthread_mutex_lock(&g_nbi_mu);
+    held_t *h = &g_held[q->ticket % NBI_SLOTS];
+    if (h->fetch && h->ticket == q->ticket && (rc || !take_held(h))) h->fetch = NULL;
+    pthread_mutex_unlock(&g_nbi_mu);
+  }
+  return rc ? engine_err(rc) : 0;
+}
+
 /* Complete the outstanding requests of one context. */
 static int nbi_quiet_list(nbi_list_t *l) {
   int rc = 0;
   for (int i = 0; i < l->n; i++) {
-    uint64_t f = 0;
-    const int r = b200shm_serve_wait(g_srv, l->v[i].ticket, 60.0, &f);
-    if (r) rc = engine_err(r);
-    else if (l->v[i].fetch) memcpy(l->v[i].fetch, &f, (size_t)l->v[i].size);
+    const int r = nbi_complete(&l->v[i]);
+    if (r) rc = r;
   }
   l->n = 0;
   return rc;
@@ -680,10 +719,18 @@ static int nbi_enqueue_on(nbi_list_t *l, const b200shm_request *r, void *fetch, 
   if (!l) return set_err(B200SHM_ERR_ARG, "invalid context");
   b200shm_server *s = job_server();
   if (!s) return 1;
-  uint64_t tk = 0;
+  nbi_t q = {UINT64_MAX, fetch != NULL};
   const double t0 = shmemx_wtime();
   for (;;) {
-    const int rc = b200shm_serve_enqueue(s, r, &tk);
+    int rc = B200SHM_ERR_BUSY;
+    pthread_mutex_lock(&g_nbi_mu);
+    held_t *h = &g_held[g_next_ticket % NBI_SLOTS];
+    if (!h->fetch || take_held(h)) {
+      rc = b200shm_serve_enqueue(s, r, &q.ticket);
+      if (q.ticket != UINT64_MAX) g_next_ticket = q.ticket + 1; /* it is in the ring */
+      if (rc == 0 && fetch) *h = (held_t){q.ticket, fetch, size};
+    }
+    pthread_mutex_unlock(&g_nbi_mu);
     if (rc == 0) break;
     if (rc != B200SHM_ERR_BUSY) return engine_err(rc);
     if (l->n) nbi_quiet_list(l); /* free slots held by this context */
@@ -693,19 +740,11 @@ static int nbi_enqueue_on(nbi_list_t *l, const b200shm_request *r, void *fetch, 
   if (l->n == l->cap) {
     const int cap = l->cap ? 2 * l->cap : 64;
     nbi_t *n = (nbi_t *)realloc(l->v, (size_t)cap * sizeof(nbi_t));
-    if (!n) {
-      uint64_t f = 0;
-      b200shm_serve_wait(s, tk, 60.0, &f);
-      if (fetch) memcpy(fetch, &f, (size_t)size);
-      return 0;
-    }
+    if (!n) return nbi_complete(&q);
     l->v = n;
     l->cap = cap;
   }
-  l->v[l->n].ticket = tk;
-  l->v[l->n].fetch = fetch;
-  l->v[l->n].size = size;
-  l->n++;
+  l->v[l->n++] = q;
   return 0;
 }
 static int nbi_enqueue(const b200shm_request *r, void *fetch, int size) {
