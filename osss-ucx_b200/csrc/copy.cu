@@ -538,12 +538,10 @@ void spread(const char *src, char *dst, uint64_t step, int P, uint64_t len, int 
    * two). */
   constexpr int kHalfSm = 100000;
   size_t smem = 0;
-  if (tiles >= 1024) {
-    static const bool ok = cudaFuncSetAttribute(k_spread<BLK>,
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                kHalfSm) == cudaSuccess;
-    if (ok) smem = kHalfSm;
-  }
+  if (tiles >= 1024 && /* the claim is the current device's: asked for on each launch */
+      cudaFuncSetAttribute(k_spread<BLK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHalfSm) ==
+          cudaSuccess)
+    smem = kHalfSm;
   k_spread<BLK><<<grid, 256, smem, s>>>(src, dst, step, P, len, nblk, mpc, skip, blk);
   count_launch();
 }
