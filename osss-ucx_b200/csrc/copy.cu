@@ -576,6 +576,32 @@ int fcollect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
   return B200SHM_OK;
 }
 
+/* Where s is being captured, the upload of a table runs at each replay of the
+ * graph: from a copy that the graph owns, not from the caller's. */
+static int table_for_graph(const std::vector<uint64_t> &pre, cudaStream_t s,
+                           const uint64_t **table) {
+  cudaStreamCaptureStatus cap;
+  cudaGraph_t graph = nullptr;
+  B200_CK(cudaStreamGetCaptureInfo(s, &cap, nullptr, &graph));
+  if (cap != cudaStreamCaptureStatusActive) return B200SHM_OK;
+  auto *own = new std::vector<uint64_t>(pre);
+  cudaUserObject_t obj;
+  cudaError_t e = cudaUserObjectCreate(
+      &obj, own, [](void *p) { delete (std::vector<uint64_t> *)p; }, 1,
+      cudaUserObjectNoDestructorSync);
+  if (e != cudaSuccess) {
+    delete own;
+    return cuda_fail(e, "collect: table of a captured call");
+  }
+  *table = own->data();
+  e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove);
+  if (e != cudaSuccess) {
+    cudaUserObjectRelease(obj, 1);
+    return cuda_fail(e, "collect: table of a captured call");
+  }
+  return B200SHM_OK;
+}
+
 int collect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint64_t src_off,
                    const uint64_t *nbytes, cudaStream_t s) {
   int rc = check_team(pe_start, pe_stride, P);
@@ -612,10 +638,11 @@ int collect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint64
   } else if (P < 1032) {
     by_value(Uneven<1032>{});
   } else {
+    const uint64_t *table = pre.data();
+    if ((rc = table_for_graph(pre, s, &table))) return rc;
     uint64_t *dev = nullptr;
     B200_CK(cudaMallocAsync((void **)&dev, pre.size() * sizeof(uint64_t), s));
-    B200_CK(cudaMemcpyAsync(dev, pre.data(), pre.size() * sizeof(uint64_t),
-                            cudaMemcpyHostToDevice, s));
+    B200_CK(cudaMemcpyAsync(dev, table, pre.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
     spread(src, dst, m.step, P, total, P, -1, Uneven<0>{dev}, s);
     B200_CK(cudaFreeAsync(dev, s));
   }
