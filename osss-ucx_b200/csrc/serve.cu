@@ -391,6 +391,22 @@ __device__ __forceinline__ void stv(char *p, T v) {
   memcpy(p, &v, sizeof(T));
 }
 
+/* A pack of sources by a plain load, as in copy_core.cuh: an earlier request
+ * of the same kernel may have written it, and this SM may have read what was
+ * there before.  The read-only path of the per-call kernels' ld_pack is for
+ * data that nothing writes while the kernel runs, and the fence that follows
+ * a claim does not order it. */
+template <class T, int V>
+__device__ __forceinline__ Pack<T, V> ld_served(const char *p) {
+  if constexpr (sizeof(Pack<T, V>) == 16) {
+    return *(const Pack<T, V> *)p;
+  } else {
+    Pack<T, V> r;
+    memcpy(&r, p, sizeof(r));
+    return r;
+  }
+}
+
 /* Where a float MIN/MAX result depends on operand order (a NaN, or both
  * zeros, among the inputs): replay the algorithm's order for element e
  * and write what each member receives (rec_dbl gives members different
@@ -450,10 +466,10 @@ __device__ Pack<T, V> tree_pack(const char *s, uint64_t step, int P, int p2s, in
       if (u < k) {
         const int q = qb + u;
         const int own = binomial ? q : (int)(((long long)q * P + p2s - 1) >> lg);
-        x[u] = ld_pack<T, V>(s + (uint64_t)own * step);
+        x[u] = ld_served<T, V>(s + (uint64_t)own * step);
         if (!binomial) {
           ex[u] = (int)(((long long)(q + 1) * P + p2s - 1) >> lg) - own == 2;
-          if (ex[u]) e[u] = ld_pack<T, V>(s + (uint64_t)(own + 1) * step);
+          if (ex[u]) e[u] = ld_served<T, V>(s + (uint64_t)(own + 1) * step);
         }
       }
     }
@@ -497,7 +513,7 @@ __device__ void reduce_units(const b200shm_request &r, const char *src0, char *d
 #pragma unroll
     for (int i = 0; i < V; i++) cls[i] = 0;
     if (chain) {
-      v = ld_pack<T, V>(s);
+      v = ld_served<T, V>(s);
       if constexpr (MM) {
 #pragma unroll
         for (int i = 0; i < V; i++) cls[i] = fclass(v.x[i]);
@@ -506,7 +522,7 @@ __device__ void reduce_units(const b200shm_request &r, const char *src0, char *d
         PK x[8];
 #pragma unroll
         for (int m = 0; m < 8; m++)
-          if (j + m < P) x[m] = ld_pack<T, V>(s + (uint64_t)(j + m) * step);
+          if (j + m < P) x[m] = ld_served<T, V>(s + (uint64_t)(j + m) * step);
 #pragma unroll
         for (int m = 0; m < 8; m++)
           if (j + m < P) {
