@@ -893,7 +893,7 @@ struct b200shm_server {
   unsigned Q = 0;
   int ctas = 0;
   cudaStream_t stream = nullptr;
-  unsigned long long tail = 0; /* next ticket */
+  std::atomic<unsigned long long> tail{0}; /* next ticket; written under mu */
   bool stopping = false;       /* stop asked: every tail written carries kStopBit */
   std::mutex mu;
 };
