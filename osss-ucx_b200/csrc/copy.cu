@@ -425,24 +425,26 @@ __global__ void __launch_bounds__(256, U > 2 ? 4 : 6)
 #pragma unroll 1
     for (int u = 0; u < U; u++) {
       const int t = tw + u * 512 + lane * 16;
-      if (w.x0 + t >= 0 && t + 16 <= end) {
-        s = w.at(col, t, &rem);
-        st16(row + t, meet16(s, s + w.jump, 0, rem < 16 ? rem : 16, 16));
-      } else if (t < end) { /* the row's ends: byte by byte */
-#pragma unroll 1
-        for (int i = 0; i < 16; i++) {
-          const int64_t y = w.x0 + t + i;
-          if (y < 0 || t + i >= end) continue;
-          const uint64_t k = (uint64_t)y / B;
-          row[t + i] = src0[j * B + k * step + ((uint64_t)y - k * B)];
-        }
+      /* at the row's ends part of a vector: its bytes [i0, i1) */
+      const int i0 = w.x0 + t < 0 ? a - t : 0;
+      const int i1 = t + 16 <= end ? 16 : (int)(end - t);
+      if (i1 <= i0) continue;
+      s = w.at(col, t + i0, &rem) - i0;
+      const uint4 x = meet16(s, s + w.jump, i0, rem < i1 - i0 ? i0 + rem : i1, i1);
+      if (i1 - i0 == 16) {
+        st16(row + t, x);
+      } else {
+        const unsigned wd[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int i = 0; i < 16; i++)
+          if (i >= i0 && i < i1) row[t + i] = (char)(wd[i >> 2] >> (8 * (i & 3)));
       }
     }
   }
 }
 
-/* alltoall of blocks of less than 16 bytes: one thread per word of the
- * flattened [pair][word] space. */
+/* alltoall of small blocks and of few words: one thread per word of the
+ * flattened [pair][word] space, in the sources' order. */
 template <class W>
 __global__ void __launch_bounds__(256) k_alltoall_flat(const char *src0, char *dst0,
                                                        uint64_t step, int P, uint64_t nw) {
@@ -663,10 +665,27 @@ int alltoall_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
   const char *sp = m.first + src_off;
   char *dp = m.first + dest_off;
   const uint64_t bits = src_off | dest_off | B;
-  if (B < 16) { /* more than two blocks may meet in a vector */
-    const uint64_t w = bits & 7 ? (bits & 3 ? 1 : 4) : 8, nw = B / w;
-    const unsigned g = grid_for((uint64_t)P * P * nw, 256, 8);
+  const uint64_t nv = (((uintptr_t)dp & 15) + (uint64_t)P * B + 15) / 16; /* vectors of a row */
+  const bool many = nv * (uint64_t)P >= 16ull * 256 * st().sm_count;
+  /* Words of the common width of blocks and offsets, one a thread, in the
+   * sources' order: for blocks of less than 16 bytes (more than two may meet
+   * in a vector), and where a step has few words, or blocks so small that
+   * most warps' vectors meet a block end.  Vectors / words in us, in a graph:
+   * words of 8 bytes, 128 members x 456 bytes 6.5 / 5.3, x 1000 10.5 / 9.9,
+   * x 2056 14.4 / 19.2, 24 x 2056 2.4 / 2.2; of 4, 128 x 36 2.5 / 2.2, x 100
+   * 3.2 / 3.3, 24 x 228 1.9 / 1.7, 48 x 388 2.3 / 2.5; of 1, 24 x 101 2.2 /
+   * 1.8, 48 x 101 2.0 / 2.5; whole vectors, 96 x 256 2.4 / 2.3, 48 x 256 1.7 /
+   * 1.8, 128 x 1008 (four a thread) 5.1 / 5.8. */
+  const uint64_t w = bits & 15 ? bits & 7 ? bits & 3 ? 1 : 4 : 8 : 16, nw = B / w;
+  const uint64_t words = (uint64_t)P * P * nw;
+  const bool flat = w == 16  ? nw >= 4 && words >= 70000 && !many
+                    : w == 8 ? nw <= 128 || words <= 200000
+                    : w == 4 ? nw <= 12 || words <= 130000
+                             : words <= 100000;
+  if (flat || B < 16) {
+    const unsigned g = grid_for(words, 256, 8);
     switch (w) {
+    case 16: k_alltoall_flat<uint4><<<g, 256, 0, s>>>(sp, dp, m.step, P, nw); break;
     case 8: k_alltoall_flat<unsigned long long><<<g, 256, 0, s>>>(sp, dp, m.step, P, nw); break;
     case 4: k_alltoall_flat<unsigned><<<g, 256, 0, s>>>(sp, dp, m.step, P, nw); break;
     default: k_alltoall_flat<unsigned char><<<g, 256, 0, s>>>(sp, dp, m.step, P, nw); break;
@@ -674,7 +693,6 @@ int alltoall_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
     count_launch();
     return B200SHM_OK;
   }
-  const uint64_t nv = (((uintptr_t)dp & 15) + (uint64_t)P * B + 15) / 16; /* vectors of a row */
   const unsigned gy = (unsigned)((uint64_t)P < kMaxGridY ? (uint64_t)P : kMaxGridY);
   auto grid = [&](int u) { return dim3((unsigned)((nv + 256 * u - 1) / (256 * u)), gy); };
   /* More vectors a thread once the grid fills the SMs four times over (below
@@ -683,9 +701,8 @@ int alltoall_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
    * long, so small blocks want short runs.  128 members, U = 1 / 2 / 4:
    * 1004 bytes 12.4 / 12.4 us, 2052 18.6 / 16.5, 4100 37.0 / 29.1 / 35.0,
    * 9999 82 / 59.5 / 68, 16388 - / 90.5 / 96.3, 24580 - / 131 / 133,
-   * 65532 (four) 321. */
-  const bool many = nv * (uint64_t)P >= 16ull * 256 * st().sm_count;
-  /* blocks no larger than a CTA's bytes divide by a reciprocal */
+   * 65532 (four) 321.  Blocks no larger than a CTA's bytes divide by a
+   * reciprocal. */
   auto recip = [&](uint64_t u) { return B <= 4096 * u ? (unsigned)((1ull << 32) / B) + 1 : 0u; };
   if ((bits & 15) == 0) {
     if (many)
