@@ -21,6 +21,8 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "copy_core.cuh"
@@ -78,11 +80,24 @@ __device__ __forceinline__ uint4 meet16(const char *s, const char *c, int i0, in
 struct Even { /* of B bytes each */
   uint64_t B;
   __device__ __forceinline__ int find(uint64_t x, int, uint64_t *b) const {
+    if ((x | B) >> 32 == 0) { /* half the instructions */
+      const unsigned k = (unsigned)x / (unsigned)B;
+      *b = (unsigned)x - k * (unsigned)B;
+      return (int)k;
+    }
     const uint64_t k = x / B;
     *b = x - k * B;
     return (int)k;
   }
   __device__ __forceinline__ uint64_t size(int) const { return B; }
+};
+struct Whole { /* one block, the row */
+  uint64_t len;
+  __device__ __forceinline__ int find(uint64_t x, int, uint64_t *b) const {
+    *b = x;
+    return 0;
+  }
+  __device__ __forceinline__ uint64_t size(int) const { return len; }
 };
 /* of uneven sizes: pre[k] = the row position of block k, pre[P] = the row's
  * length.  The table is the kernel's parameter (N entries at most), read
@@ -115,6 +130,7 @@ struct Table {
   __device__ __forceinline__ uint64_t size(int k) const { return t.pre[k + 1] - t.pre[k]; }
 };
 __device__ __forceinline__ Even blocks(const Even &e) { return e; }
+__device__ __forceinline__ Whole blocks(const Whole &w) { return w; }
 template <int N>
 __device__ __forceinline__ Table<N> blocks(const Uneven<N> &t) {
   return Table<N>{t};
@@ -196,6 +212,39 @@ __global__ void __launch_bounds__(256, 6) k_spread(const char *src0, char *dst0,
 #pragma unroll
         for (int i = 0; i < 16; i++)
           if (i >= e0 && i < e1) d[(uint64_t)j * step + i] = (char)(w[i >> 2] >> (8 * (i & 3)));
+  }
+}
+
+/* Short rows: one thread per byte of the row.  What bounds them is the launch
+ * and one round of loads, and there is no vector to put together first (3 us
+ * in a graph for 8 members x 4 bytes by k_spread, 1.5 this way). */
+template <class BLK>
+__global__ void __launch_bounds__(256) k_spread_bytes(const char *src0, char *dst0, uint64_t step,
+                                                      int P, uint64_t len, int nblk, int mpc,
+                                                      int skip, const __grid_constant__ BLK prm) {
+  const auto blk = blocks(prm);
+  const uint64_t x = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+  if (x >= len) return;
+  uint64_t b;
+  const int k = blk.find(x, nblk, &b);
+  const char c = src0[(uint64_t)k * step + b];
+  const int j0 = blockIdx.y * mpc, j1 = j0 + mpc < P ? j0 + mpc : P;
+  char *d = dst0 + x + (uint64_t)j0 * step;
+  for (int j = j0; j < j1; j++, d += step)
+    if (j != skip) *d = c;
+}
+
+/* broadcast of aligned rows to few members: neighbouring vectors by a grid
+ * that strides, each written to every member (but the root).  For broadcasts
+ * that stay in L2, and to one member, where nothing pays for k_spread's
+ * setting up of each vector. */
+__global__ void __launch_bounds__(256) k_broadcast(const char *src, char *dst0, uint64_t step,
+                                                   int P, int root, uint64_t n) {
+  for (uint64_t v = (uint64_t)blockIdx.x * 256 + threadIdx.x; v < n;
+       v += (uint64_t)gridDim.x * 256) {
+    const uint4 u = ld16(src + v * 16);
+    for (int j = 0; j < P; j++)
+      if (j != root) st16(dst0 + (uint64_t)j * step + v * 16, u);
   }
 }
 
@@ -523,24 +572,50 @@ unsigned x_blocks(uint64_t n, uint64_t ypairs, uint64_t want) {
   return (unsigned)(per < 1 ? 1 : per);
 }
 
-/* Launch k_spread over a row of len bytes: rows of few vectors split their
- * members over more CTAs, so that the grid fills the SMs. */
+/* Launch the copy of a row of len bytes to P members; grid16: its blocks and
+ * the offsets are multiples of 16. */
 template <class BLK>
 void spread(const char *src, char *dst, uint64_t step, int P, uint64_t len, int nblk, int skip,
-            const BLK &blk, cudaStream_t s) {
+            bool grid16, const BLK &blk, cudaStream_t s) {
+  const uint64_t sms = (uint64_t)st().sm_count;
+  auto members_per_cta = [&](uint64_t split, uint64_t least) {
+    split = std::max<uint64_t>(1, std::min<uint64_t>(split, ((uint64_t)P + least - 1) / least));
+    return (int)((P + split - 1) / split);
+  };
+  /* Bytes against vectors, us in a graph: fcollect of 32 x 100 bytes 1.6 / 1.9,
+   * 16 x 260 1.7 / 1.9, 6 x 4100 1.6 / 2.2, 128 x 64 (whole vectors) 1.8 / 1.9; a
+   * broadcast of 4096 to 4 1.6 either way; an uneven collect, whose table every
+   * byte searches, of 4 members and 129 KB 2.0 / 1.8. */
+  constexpr bool table = !std::is_same<BLK, Even>::value && !std::is_same<BLK, Whole>::value;
+  if (len <= (grid16 ? 1024 : 8192) || (!grid16 && !table && len * (uint64_t)P <= 1 << 20)) {
+    const uint64_t gx = (len + 255) / 256;
+    const int mpc = members_per_cta(2 * sms / gx, 2);
+    k_spread_bytes<BLK><<<dim3((unsigned)gx, (unsigned)((P + mpc - 1) / mpc)), 256, 0, s>>>(
+        src, dst, step, P, len, nblk, mpc, skip, blk);
+    count_launch();
+    return;
+  }
+  /* The members are split over more CTAs where the row's vectors leave SMs
+   * idle: short rows, two members to a CTA at least, into one wave of the six
+   * CTAs an SM holds (128 x 260 bytes 2.9 us, 4.5 in the 1.3 waves that eight
+   * an SM make), longer ones, four to a CTA, into eight an SM (128 x 8 KiB 21.9
+   * against 24.6, 32 x 64 KiB 10.6 against 12.1: the SMs finish more evenly; 8 x
+   * 64 KiB 2.3, with two to a CTA 2.6). */
   const uint64_t tiles = (((uintptr_t)dst & 15) + len + 4095) / 4096;
-  uint64_t split = (8ull * st().sm_count + tiles - 1) / tiles;
-  if (split > (uint64_t)P) split = (uint64_t)P;
-  const int mpc = (int)((P + split - 1) / split);
+  const int mpc = tiles < 128 ? members_per_cta(6 * sms / tiles, 2)
+                              : members_per_cta((8 * sms + tiles - 1) / tiles, 4);
   dim3 grid((unsigned)tiles, (unsigned)((P + mpc - 1) / mpc));
-  /* Long rows run two CTAs an SM, by a claim on shared memory: fewer rows
-   * are written at a time, which DRAM likes better (128 members x 32 KiB:
-   * 80.5 us with two, 82.5 with three, 85.9 with six).  Rows of fewer
-   * vectors want the CTAs (32 members x 32 KiB: 8.3 us with six, 9.4 with
-   * two). */
+  /* Long rows of many members run two CTAs an SM, by a claim on shared
+   * memory: fewer rows are written at a time, which DRAM likes better.  Two /
+   * six CTAs, us in a graph: 128 members, 512 tiles 39.9 / 42.4, 1024 76.3 /
+   * 81.2; 64 members, 512 20.8 / 21.9; 32 members, 512 10.7 / 10.6, 768 15.4 /
+   * 15.7, an uneven collect of 512 11.4 / 10.8, 640 13.0 / 13.1; 16 members, 1024
+   * 40.5 / 46; but a broadcast of 4096 tiles to 8 19.5 / 19.0, of 16384 100 / 84, to
+   * 4 72 / 42.  (A resident serving loop leaves room for one such CTA an SM,
+   * and takes nothing: 128 x 32 KiB 78.0 beside it, 82.8 with six.) */
   constexpr int kHalfSm = 100000;
   size_t smem = 0;
-  if (tiles >= 1024 && /* the claim is the current device's: asked for on each launch */
+  if (tiles >= 640 && P >= 16 && /* the claim is the current device's: asked for on each launch */
       cudaFuncSetAttribute(k_spread<BLK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHalfSm) ==
           cudaSuccess)
     smem = kHalfSm;
@@ -573,7 +648,7 @@ int fcollect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
     count_launch();
     return B200SHM_OK;
   }
-  spread(m.first + src_off, m.first + dest_off, m.step, P, nbytes * (uint64_t)P, P, -1,
+  spread(m.first + src_off, m.first + dest_off, m.step, P, nbytes * (uint64_t)P, P, -1, vec,
          Even{nbytes}, s);
   return B200SHM_OK;
 }
@@ -633,7 +708,7 @@ int collect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint64
    * kernel); teams too large for one keep it in device memory. */
   auto by_value = [&](auto blk) {
     memcpy(blk.pre, pre.data(), pre.size() * sizeof(uint64_t));
-    spread(src, dst, m.step, P, total, P, -1, blk, s);
+    spread(src, dst, m.step, P, total, P, -1, false, blk, s);
   };
   if (P < 136) {
     by_value(Uneven<136>{});
@@ -645,7 +720,7 @@ int collect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint64
     uint64_t *dev = nullptr;
     B200_CK(cudaMallocAsync((void **)&dev, pre.size() * sizeof(uint64_t), s));
     B200_CK(cudaMemcpyAsync(dev, table, pre.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
-    spread(src, dst, m.step, P, total, P, -1, Uneven<0>{dev}, s);
+    spread(src, dst, m.step, P, total, P, -1, false, Uneven<0>{dev}, s);
     B200_CK(cudaFreeAsync(dev, s));
   }
   return B200SHM_OK;
@@ -790,8 +865,20 @@ int broadcast_launch(int root, int pe_start, int pe_stride, int P, uint64_t dest
     return fail(B200SHM_ERR_ARG, "broadcast: dest and source overlap");
   if (nbytes == 0 || P == 1) return B200SHM_OK;
   Members m = members(pe_start, pe_stride, P);
-  spread(m.first + (uint64_t)root * m.step + src_off, m.first + dest_off, m.step, P, nbytes, 1,
-         root, Even{nbytes}, s);
+  const char *from = m.first + (uint64_t)root * m.step + src_off;
+  const bool vec = ((src_off | dest_off | nbytes) & 15u) == 0;
+  /* us in a graph, k_broadcast / k_spread (without its claim): to one member
+   * 4 MiB 2.4 / 3.0, 64 MiB 18 / 28; to 3 1 MiB 2.0 / 2.5, 16 MiB 9.3 / 8.5; to 7 64
+   * KiB 1.9 / 1.8, 1 MiB 2.6 / 3.0, 4 MiB 5.8 / 6.0, 16 MiB 25 / 19; to 15 1 MiB
+   * 3.8 / 4.2; to 31 1 MiB 6.3 / 6.3. */
+  const bool in_l2 = P <= 16 && nbytes >= (128 << 10) && nbytes * (uint64_t)P <= (32ull << 20);
+  if (vec && (P == 2 || in_l2)) {
+    k_broadcast<<<grid_for(nbytes / 16, 256, 8), 256, 0, s>>>(from, m.first + dest_off, m.step, P,
+                                                             root, nbytes / 16);
+    count_launch();
+    return B200SHM_OK;
+  }
+  spread(from, m.first + dest_off, m.step, P, nbytes, 1, root, vec, Whole{nbytes}, s);
   return B200SHM_OK;
 }
 
