@@ -234,7 +234,10 @@ struct Lane {
  * lane of a tree holds -- 2, 4, 8: all loaded at once; 16 to 128: chunks of 8;
  * 0: any number of chunks of 8, a binary counter over them; kRagged<L>:
  * fewer than 2^L leaves, not a power of two (a binomial tree in one lane):
- * chunks of 8, then the last leaves one by one.
+ * chunks of 8, then the last leaves one by one.  Chains: 0 where one lane
+ * has all members, so that the loop's bounds are the same in all lanes and
+ * slots beyond them cost nothing (f64 SUM in a linear order over 64 members x
+ * 409600 93 -> 72 us, int16 SUM over 2 x 2^24 50 -> 33 us), else 1.
  * True for a MIN/MAX column whose bits depend on operand order: its dests
  * are left for the exact replay. */
 template <int LEVELS>
@@ -258,10 +261,11 @@ __device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, ui
   unsigned cls = 0;
   if (live) {
     if constexpr (ORDER == ORD_CHAIN) {
-      const char *p = src + (uint64_t)l0 * a.sstep;
+      constexpr bool kOne = C == 0; /* one lane: bounds that the whole launch shares */
+      const char *p = src + (kOne ? 0 : (uint64_t)l0 * a.sstep);
       r = ld_col<T, V, MODE>(p);
-      unsigned j = (unsigned)l0 + 1; /* l1 may be the largest int: j + 8 is above it */
-      const unsigned end = (unsigned)l1;
+      unsigned j = kOne ? 1 : (unsigned)l0 + 1; /* end may be the largest int: j + 8 is above */
+      const unsigned end = (unsigned)(kOne ? P : l1);
       do { /* once at least: a MIN/MAX lane looks at its first operand below the loads */
         PK x[8];
         const uint64_t step = opaque(a.sstep);
@@ -270,7 +274,7 @@ __device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, ui
           if (j + u < end) x[u] = ld_col<T, V, MODE>(p + (uint64_t)(u + 1) * step);
         p += 8 * step;
         if constexpr (MM)
-          if (j == (unsigned)l0 + 1) cls = mm_flags<OP>(r);
+          if (j == (kOne ? 1 : (unsigned)l0 + 1)) cls = mm_flags<OP>(r);
 #pragma unroll
         for (int u = 0; u < 8; u++)
           if (j + u < end) {
@@ -356,6 +360,11 @@ __device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, ui
         }
       } else {
         constexpr bool kRest = C < 0;
+        /* the last leaves of a complex PROD tree one by one: seven at a time
+         * take registers the products need (complex float over 15 members x
+         * 10^6 86 us, 79 so) */
+        constexpr bool kOneByOne = C < -3 && OP == B200SHM_PROD &&
+                                   (std::is_same<T, cf32>::value || std::is_same<T, cf64>::value);
         constexpr int LV = kRest ? -C : kMaxLevels - 3; /* levels of 2^k leaves (chunks) */
         PK stk[LV];
         const int n = l1 - l0;
@@ -374,13 +383,18 @@ __device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, ui
         if constexpr (LV > 3)
           for (; q + 8 <= n; q += 8) push(chunk(l0 + q, k8{}), kRest ? 3 : 0);
         if constexpr (kRest) {
-          PK x[7];
+          if constexpr (kOneByOne) {
+#pragma unroll 1
+            for (; q < n; q++) push(ld_col<T, V, MODE>(src + (uint64_t)q * a.sstep), 0);
+          } else {
+            PK x[7];
 #pragma unroll
-          for (int u = 0; u < 7; u++)
-            if (q + u < n) x[u] = ld_col<T, V, MODE>(src + (uint64_t)(q + u) * a.sstep);
+            for (int u = 0; u < 7; u++)
+              if (q + u < n) x[u] = ld_col<T, V, MODE>(src + (uint64_t)(q + u) * a.sstep);
 #pragma unroll
-          for (int u = 0; u < 7; u++)
-            if (q + u < n) push(x[u], 0);
+            for (int u = 0; u < 7; u++)
+              if (q + u < n) push(x[u], 0);
+          }
           bool have = false;
 #pragma unroll
           for (int L = 0; L < LV; L++)
@@ -460,22 +474,48 @@ __device__ __forceinline__ void reduce_edges(const RArgs &a, const Lane &ln, int
   }
 }
 
-/* CTAs per SM an instance is held to, at least: 5 (48 registers) where it
- * fits without spills (trees, chains of 8-byte elements), 4 with 4-byte
- * elements or with edges (the code for single elements costs registers, so
- * rows of whole packs, nedge == 0, have an instance without it), 2 with
- * smaller elements (unpacked into a register each); 3 for the MIN/MAX ones:
- * holding those to 64 registers (4 CTAs per SM, no spills) measured slower
- * on the 64-PE headline (f64 MAX 5908-5912 against 5938-5950 GB/s). */
-template <class T, int ORDER, bool MM, int C, bool POW2, int MODE, bool EDGES>
+/* CTAs per SM an instance is held to, at least, by what its op needs (in
+ * parentheses: the registers that leaves):
+ *   trees over power-of-two teams 5 (48), with edges or long runs 4 (64: the
+ *   code for single elements costs registers, so rows of whole packs, nedge
+ *   == 0, have an instance without it), with extra members 3 (80), with a
+ *   stack 2;
+ *   complex PROD, four temporaries an element: 4 up to 16 leaves, 3 at 32
+ *   (64 members x 409600 complex float: 76 us; 84 at 48 registers, which
+ *   spills, 91 at 84, two CTAs), 2 beyond;
+ *   chains in one lane as many as at the widths below, chains in several
+ *   lanes 5 for 8-byte elements, 4 for their MIN/MAX (a compare and two
+ *   selects) and for 4-byte ones, 3 for MIN/MAX/PROD of 2-byte elements, 2
+ *   for the others of 2 bytes and for bytes (which are unpacked into a
+ *   register each: bytes' MIN/MAX and bit operations spill 180 to 420 bytes
+ *   there, and still ran 1.1 to 3 times as fast as the one CTA of 160 to 200
+ *   registers that does not, over 24 to 256 members);
+ *   3 for the float MIN/MAX ones: holding those to 64 registers (4 CTAs, no
+ *   spills) measured slower on the 64-PE headline (f64 MAX 5908-5912 against
+ *   5938-5950 GB/s). */
+template <class T, int OP, int ORDER, bool MM, int C, bool POW2, int MODE, bool EDGES>
 constexpr int min_ctas() {
+  constexpr bool order = OP == B200SHM_MIN || OP == B200SHM_MAX, prod = OP == B200SHM_PROD;
+  constexpr bool cplx = std::is_same<T, cf32>::value || std::is_same<T, cf64>::value;
+  constexpr int es = (int)sizeof(T);
   if (MODE == kBytes) return 1;
   if (MM) return 3;
-  if (ORDER == ORD_CHAIN) return sizeof(T) < 4 ? 2 : sizeof(T) == 4 || EDGES ? 4 : 5;
-  return C == 0 || C < -3 ? 2 : !POW2 ? 3 : EDGES || C > 32 ? 4 : 5;
+  if (ORDER == ORD_CHAIN && C == 0) {
+    if (es == 1) return prod || OP == B200SHM_SUM ? 2 : 1;
+    if (es == 2) return order || prod ? 3 : 2;
+    if (std::is_same<T, f80>::value) return 1;
+    return es == 4 || std::is_same<T, cf32>::value || (cplx && prod) ? 3 : 4;
+  }
+  if (ORDER == ORD_CHAIN) {
+    if (es < 4) return es == 2 && (order || prod) ? 3 : 2;
+    return es == 4 || EDGES || order ? 4 : 5;
+  }
+  if (C == 0 || C < -3) return 2;
+  if (cplx && prod) return C > 32 ? 2 : !POW2 || C == 32 || C < 0 ? 3 : 4;
+  return !POW2 ? 3 : EDGES || C > 32 ? 4 : 5;
 }
 template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2, int MODE, bool EDGES>
-__global__ void __launch_bounds__(256, min_ctas<T, ORDER, MM, C, POW2, MODE, EDGES>())
+__global__ void __launch_bounds__(256, min_ctas<T, OP, ORDER, MM, C, POW2, MODE, EDGES>())
 k_reduce(const __grid_constant__ RArgs a) {
   const int lane = threadIdx.x & 31, lgG = ORDER == ORD_CHAIN && C == 0 ? 0 : a.lgG;
   Lane ln;
@@ -539,13 +579,14 @@ int resident_ctas(const void *kernel) {
 
 /* Launch over `lanes` threads of work.  Grid: up to 8 waves of the CTAs one
  * SM holds at once (B200SHM_REDUCE_WAVES overrides it, or
- * B200SHM_REDUCE_CTAS_PER_SM gives a fixed count).  On the 64-PE x 2^20
+ * B200SHM_REDUCE_CTAS_PER_SM gives a fixed count); for chains in one lane 8
+ * CTAs an SM (8 members x 2^21 int32: 19.6 us, 21.3 with 8 waves).  On the 64-PE x 2^20
  * workload one exact wave was slowest (5.27 TB/s over the six reductions):
  * CTAs of a grid-stride loop finish unevenly and leave their SM's slots
  * idle, while the CTAs of later waves backfill them.  4 waves gave 5.73,
  * 6-16 waves 5.78-5.80, one pack per lane 5.76.  CTAs of 256 threads, less
  * where that leaves SMs without one. */
-template <class K>
+template <bool ONE_LANE, class K>
 void launch_one(K kernel, uint64_t lanes, cudaStream_t s, const RArgs &a) {
   static int per_sm_env = -1, waves = 8;
   if (per_sm_env < 0) {
@@ -557,7 +598,9 @@ void launch_one(K kernel, uint64_t lanes, cudaStream_t s, const RArgs &a) {
   const uint64_t sms = (uint64_t)grid_sms();
   int threads = 256;
   while (threads > 64 && lanes < sms * (uint64_t)threads) threads >>= 1;
-  const int per_sm = per_sm_env ? per_sm_env : waves * resident_ctas((const void *)kernel);
+  const int per_sm = per_sm_env ? per_sm_env
+                     : ONE_LANE ? 8
+                                : waves * resident_ctas((const void *)kernel);
   kernel<<<grid_for(lanes, threads, per_sm), threads, 0, s>>>(a);
   count_launch();
 }
@@ -565,13 +608,14 @@ void launch_one(K kernel, uint64_t lanes, cudaStream_t s, const RArgs &a) {
 /* the instance with or without edges */
 template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2, int MODE>
 void launch_edges(uint64_t lanes, cudaStream_t s, const RArgs &a) {
+  constexpr bool one = ORDER == ORD_CHAIN && C == 0;
   if constexpr (V > 1) {
     if (a.nedge) {
-      launch_one(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, true>, lanes, s, a);
+      launch_one<one>(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, true>, lanes, s, a);
       return;
     }
   }
-  launch_one(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, false>, lanes, s, a);
+  launch_one<one>(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, false>, lanes, s, a);
 }
 
 /* Whether a lane has instances of 64 and 128 leaves (not long double, whose
@@ -604,9 +648,10 @@ void launch_tree(int n, uint64_t lanes, cudaStream_t s, const RArgs &a) {
  * member, 2.82 TB/s, at 2 of 128 5.50; 128 members at 4 of 32 4.89, at 2 of
  * 64 5.70; but 128 to 255 members with extras or edges at 2 lanes 1-8 %
  * slower.)  Long runs only where at least 256 threads an SM are left: 256
- * members x 65536 at 4 of 64 4.36 TB/s, at 8 of 32 2.6.  On the 64-PE workload G = 2 with 32 leaves per lane ran the f32 tree at 5.6-5.9 TB/s,
- * G = 4 with 16 at 5.2-5.4 (a warp then reads 128 rather than 256
- * consecutive bytes of each member per load).  Few columns: what counts is
+ * members x 65536 at 4 of 64 4.36 TB/s, at 8 of 32 2.6.  On the 64-PE
+ * workload G = 2 with 32 leaves per lane ran the f32 tree at 5.6-5.9 TB/s, G =
+ * 4 with 16 at 5.2-5.4 (a warp then reads 128 rather than 256 consecutive
+ * bytes of each member per load).  Few columns: what counts is
  * how many rounds of loads a lane makes in turn, so lanes are added while a
  * lane holds more than 4 leaves and the columns are fewer than 128 per SM
  * over G^2 (each doubling halves the run of each member that a warp reads,
@@ -648,8 +693,11 @@ void run_mode(RArgs &a, cudaStream_t s) {
   const int run = long_runs ? 128 : 32;
   a.lgG = split ? lanes_log2<ORDER>(a.nvec + a.nedge, leaves, sizeof(T) == 16, run) : 0;
   const uint64_t lanes = std::max<uint64_t>(a.nvec + a.nedge, 1) << a.lgG;
-  if constexpr (ORDER == ORD_CHAIN) {
-    launch_edges<T, OP, ORDER, V, MM, 1, true, MODE>(lanes, s, a);
+  if constexpr (ORDER == ORD_CHAIN && any_order) {
+    if (MM || a.lgG) launch_edges<T, OP, ORDER, V, MM, 1, true, MODE>(lanes, s, a);
+    else if constexpr (!MM) launch_edges<T, OP, ORDER, V, MM, 0, true, MODE>(lanes, s, a);
+  } else if constexpr (ORDER == ORD_CHAIN) {
+    launch_edges<T, OP, ORDER, V, MM, 0, true, MODE>(lanes, s, a);
   } else if constexpr (ORDER == ORD_BINOMIAL) {
     if (pow2) launch_tree<T, OP, ORDER, V, true, MODE>(leaves >> a.lgG, lanes, s, a);
     else if (P < 8) launch_edges<T, OP, ORDER, V, false, kRagged<3>, false, MODE>(lanes, s, a);
