@@ -72,16 +72,15 @@ namespace {
 /* Teams of more than 2 * kExactLeaves - 1 members only (smaller ones replay
  * such elements inside the streaming kernel, exact_columns): second pass
  * over the elements the streaming kernel deferred (it left their dests
- * untouched, so in-place sources are still intact): one CTA
- * per element stages the P inputs in shared memory, then replays the
- * algorithm's operand order from there.  (Launched as a programmatic
+ * untouched, so in-place sources are still intact): one CTA per element
+ * stages the P inputs in shared memory, then replays the algorithm's
+ * operand order from there.  (Launched as a programmatic
  * dependent of the streaming kernel, its CTAs became resident on the few SMs
  * that kernel left free and stayed there: 256 members x 20000 floats with
  * NaNs throughout ran 16.1 ms, 5.8 as an ordinary launch; without any, 33.2
  * us either way.)  The last CTA to leave sets the counter back to zero for
- * the next call
- * (every CTA reads it before it counts itself out), so no memset precedes
- * the streaming kernel. */
+ * the next call (every CTA reads it before it counts itself out), so no
+ * memset precedes the streaming kernel. */
 template <class T, int OP>
 __global__ void __launch_bounds__(256) k_minmax_fix(const RArgs a,
                                                     const unsigned long long *list,
@@ -147,12 +146,14 @@ __global__ void __launch_bounds__(256) k_minmax_fix(const RArgs a,
  * How a column is accessed (MODE):
  *   kPacks    16-byte accesses: every row has the same offset from the
  *             16-byte grid, so the columns begin at the grid's first point
- *             in the rows and the elements before it and after the last
- *             whole pack (at most 2(V-1)) are columns of one element, in
- *             the same launch;
+ *             in the dest rows (rows of 4 KiB or more: at the first 128-byte
+ *             line) and the elements before it (fewer than a line's) and
+ *             after the last whole pack (at most V - 1) are columns of one
+ *             element, in the same launch;
  *   kElements one element each, at its own alignment: rows of different
  *             offsets (dest and source shifted against each other, member
- *             strides off the grid);
+ *             strides off the grid), and few elements of 1 or 2 bytes off
+ *             the grid;
  *   kBytes    elements at any byte offset. */
 enum { kPacks = 0, kElements = 1, kBytes = 2 };
 
@@ -719,7 +720,11 @@ int run(const RArgs &base, cudaStream_t s) {
   const uintptr_t sp = (uintptr_t)a.src, dp = (uintptr_t)a.dst;
   a.head = 0;
   if (!MM || a.p2s <= kExactLeaves) a.fix_list = nullptr;
-  if (((sp ^ dp) & 15) == 0 && (steps & 15) == 0 && dp % sizeof(T) == 0) {
+  /* few narrow elements off the grid: what counts is lanes, and an element a
+   * lane makes V times as many (bytes, MAX over 8 members x 8193: 2.1 us, 3.8
+   * in packs; over 2 x 32769 2.0 and 2.6; 8 x 524289 the other way round) */
+  const bool few = sizeof(T) <= 2 && (dp & 15) && a.N <= 65536;
+  if (((sp ^ dp) & 15) == 0 && (steps & 15) == 0 && dp % sizeof(T) == 0 && !few) {
     /* the packs begin at a 128-byte line of the dest, so that warps do not
      * share lines (vectors shorter than a few lines: at the 16-byte grid) */
     const uintptr_t grid = sizeof(T) < 16 && a.N * sizeof(T) >= 4096 ? 128 : 16;
