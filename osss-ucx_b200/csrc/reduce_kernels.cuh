@@ -361,11 +361,12 @@ __device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, ui
         }
       } else {
         constexpr bool kRest = C < 0;
-        /* the last leaves of a complex PROD tree one by one: seven at a time
-         * take registers the products need (complex float over 15 members x
-         * 10^6 86 us, 79 so) */
-        constexpr bool kOneByOne = C < -3 && OP == B200SHM_PROD &&
-                                   (std::is_same<T, cf32>::value || std::is_same<T, cf64>::value);
+        /* the last leaves of complex PROD and long double trees one by one:
+         * seven at a time take registers the operation needs (complex float
+         * PROD over 15 members x 10^6 86 us, 79 so) */
+        constexpr bool kOneByOne =
+            C < -3 && (std::is_same<T, f80>::value ||
+                       (OP == B200SHM_PROD && !std::is_floating_point<T>::value));
         constexpr int LV = kRest ? -C : kMaxLevels - 3; /* levels of 2^k leaves (chunks) */
         PK stk[LV];
         const int n = l1 - l0;
@@ -499,12 +500,11 @@ constexpr int min_ctas() {
   constexpr bool order = OP == B200SHM_MIN || OP == B200SHM_MAX, prod = OP == B200SHM_PROD;
   constexpr bool cplx = std::is_same<T, cf32>::value || std::is_same<T, cf64>::value;
   constexpr int es = (int)sizeof(T);
-  if (MODE == kBytes) return 1;
+  if (MODE == kBytes && (es < 16 || MM)) return 1;
   if (MM) return 3;
   if (ORDER == ORD_CHAIN && C == 0) {
     if (es == 1) return prod || OP == B200SHM_SUM ? 2 : 1;
     if (es == 2) return order || prod ? 3 : 2;
-    if (std::is_same<T, f80>::value) return 1;
     return es == 4 || std::is_same<T, cf32>::value || (cplx && prod) ? 3 : 4;
   }
   if (ORDER == ORD_CHAIN) {
@@ -513,7 +513,7 @@ constexpr int min_ctas() {
   }
   if (C == 0 || C < -3) return 2;
   if (cplx && prod) return C > 32 ? 2 : !POW2 || C == 32 || C < 0 ? 3 : 4;
-  return !POW2 ? 3 : EDGES || C > 32 ? 4 : 5;
+  return !POW2 ? 3 : EDGES || C > 32 || MODE == kBytes ? 4 : 5;
 }
 template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2, int MODE, bool EDGES>
 __global__ void __launch_bounds__(256, min_ctas<T, OP, ORDER, MM, C, POW2, MODE, EDGES>())
@@ -626,7 +626,8 @@ constexpr bool kLongRuns = MODE == kPacks && !std::is_same<T, f80>::value;
 /* leaves per lane n -> the instance */
 template <class T, int OP, int ORDER, int V, bool POW2, int MODE>
 void launch_tree(int n, uint64_t lanes, cudaStream_t s, const RArgs &a) {
-  constexpr int C16 = MODE == kPacks ? 16 : 0, C32 = MODE == kPacks ? 32 : 0;
+  constexpr bool wide = MODE == kPacks || sizeof(T) == 16;
+  constexpr int C16 = wide ? 16 : 0, C32 = wide ? 32 : 0;
   constexpr int C64 = kLongRuns<T, MODE> ? 64 : 0, C128 = kLongRuns<T, MODE> ? 128 : 0;
   switch (n) {
   case 2: launch_edges<T, OP, ORDER, V, false, 2, POW2, MODE>(lanes, s, a); break;
