@@ -136,20 +136,40 @@ __device__ __forceinline__ Table<N> blocks(const Uneven<N> &t) {
   return Table<N>{t};
 }
 
+/* The copy of a row of len bytes, nblk blocks, from src0 on to P members'
+ * dests from dst0 on, mpc members a CTA, all but `skip`.  Padded to 32 bytes
+ * past a multiple of 64: a launch takes the host least with so many bytes of
+ * parameters (an empty kernel: 2.05 us at 32, 96, 160, 224, 288 or 1120 bytes, 2.4
+ * within 8 of these, 2.7 elsewhere; fcollect of 8 x 128 bytes, a call from
+ * Python: 3.9 us with 72 bytes, 3.2 with 96). */
+template <class BLK>
+struct Row {
+  const char *src0;
+  char *dst0;
+  uint64_t step, len;
+  int P, nblk, mpc, skip;
+  BLK prm;
+  char pad[(32 + 64 - (48 + sizeof(BLK)) % 64) % 64];
+};
+static_assert(sizeof(Row<Even>) % 64 == 32 && sizeof(Row<Uneven<136>>) % 64 == 32, "see above");
+
 /* fcollect, collect and broadcast: every member's dest row is the same
  * `len` bytes, the blocks one after the other (fcollect.c:370-403,
  * collect.c:35-591).  One thread per 16-byte vector of the row: it puts the
  * vector together once and writes it into the members of its blockIdx.y
  * (all but `skip`).  Bound by the writes, P per vector read; streaming
- * stores, since this kernel does not read them again.  128 members x 32 KiB:
- * 92.4 us with one pass per source member and six CTAs an SM, 80.3 now (6.7
- * TB/s); x 32764 bytes, then 4-byte words: 274 -> 81.4; collect of 64 members
- * x 32 KiB on average, 4-byte words and an uploaded table: 40.7 -> 24.5. */
+ * stores, since this kernel does not read them again.  In a graph, 128
+ * members x 32 KiB: 88.3 us with one pass per source member and six CTAs an
+ * SM, 76.2 now (91.8 and 82.4 a call in a row); x 32764 bytes, then 4-byte
+ * words: 278 -> 76.6; a collect of 64 members x 32 KiB on average, a call in a
+ * row, 4-byte words and an uploaded table: 45.5 -> 24.5. */
 template <class BLK>
-__global__ void __launch_bounds__(256, 6) k_spread(const char *src0, char *dst0, uint64_t step,
-                                                int P, uint64_t len, int nblk, int mpc, int skip,
-                                                const __grid_constant__ BLK prm) {
-  const auto blk = blocks(prm);
+__global__ void __launch_bounds__(256, 6) k_spread(const __grid_constant__ Row<BLK> r) {
+  const auto blk = blocks(r.prm);
+  const char *const src0 = r.src0;
+  char *const dst0 = r.dst0;
+  const uint64_t step = r.step, len = r.len;
+  const int P = r.P, nblk = r.nblk, mpc = r.mpc, skip = r.skip;
   const int a = (int)((uintptr_t)dst0 & 15); /* the row begins at byte a of vector 0 */
   const int64_t x0 = ((int64_t)blockIdx.x * 256 + threadIdx.x) * 16 - a;
   const int i0 = x0 < 0 ? a : 0;
@@ -219,19 +239,17 @@ __global__ void __launch_bounds__(256, 6) k_spread(const char *src0, char *dst0,
  * and one round of loads, and there is no vector to put together first (3 us
  * in a graph for 8 members x 4 bytes by k_spread, 1.5 this way). */
 template <class BLK>
-__global__ void __launch_bounds__(256) k_spread_bytes(const char *src0, char *dst0, uint64_t step,
-                                                      int P, uint64_t len, int nblk, int mpc,
-                                                      int skip, const __grid_constant__ BLK prm) {
-  const auto blk = blocks(prm);
+__global__ void __launch_bounds__(256) k_spread_bytes(const __grid_constant__ Row<BLK> r) {
+  const auto blk = blocks(r.prm);
   const uint64_t x = (uint64_t)blockIdx.x * 256 + threadIdx.x;
-  if (x >= len) return;
+  if (x >= r.len) return;
   uint64_t b;
-  const int k = blk.find(x, nblk, &b);
-  const char c = src0[(uint64_t)k * step + b];
-  const int j0 = blockIdx.y * mpc, j1 = j0 + mpc < P ? j0 + mpc : P;
-  char *d = dst0 + x + (uint64_t)j0 * step;
-  for (int j = j0; j < j1; j++, d += step)
-    if (j != skip) *d = c;
+  const int k = blk.find(x, r.nblk, &b);
+  const char c = r.src0[(uint64_t)k * r.step + b];
+  const int j0 = blockIdx.y * r.mpc, j1 = j0 + r.mpc < r.P ? j0 + r.mpc : r.P;
+  char *d = r.dst0 + x + (uint64_t)j0 * r.step;
+  for (int j = j0; j < j1; j++, d += r.step)
+    if (j != r.skip) *d = c;
 }
 
 /* broadcast of aligned rows to few members: neighbouring vectors by a grid
@@ -591,7 +609,7 @@ void spread(const char *src, char *dst, uint64_t step, int P, uint64_t len, int 
     const uint64_t gx = (len + 255) / 256;
     const int mpc = members_per_cta(2 * sms / gx, 2);
     k_spread_bytes<BLK><<<dim3((unsigned)gx, (unsigned)((P + mpc - 1) / mpc)), 256, 0, s>>>(
-        src, dst, step, P, len, nblk, mpc, skip, blk);
+        Row<BLK>{src, dst, step, len, P, nblk, mpc, skip, blk, {}});
     count_launch();
     return;
   }
@@ -619,7 +637,7 @@ void spread(const char *src, char *dst, uint64_t step, int P, uint64_t len, int 
       cudaFuncSetAttribute(k_spread<BLK>, cudaFuncAttributeMaxDynamicSharedMemorySize, kHalfSm) ==
           cudaSuccess)
     smem = kHalfSm;
-  k_spread<BLK><<<grid, 256, smem, s>>>(src, dst, step, P, len, nblk, mpc, skip, blk);
+  k_spread<BLK><<<grid, 256, smem, s>>>(Row<BLK>{src, dst, step, len, P, nblk, mpc, skip, blk, {}});
   count_launch();
 }
 
@@ -703,9 +721,9 @@ int collect_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint64
   Members m = members(pe_start, pe_stride, P);
   const char *src = m.first + src_off;
   char *dst = m.first + dest_off;
-  /* The table of positions as a kernel parameter (64 members x 32 KiB on
-   * average: 46 us with an allocation, an upload and a free around the
-   * kernel); teams too large for one keep it in device memory. */
+  /* The table of positions as a kernel parameter, which takes an allocation,
+   * an upload and a free from around the kernel; teams too large for one keep
+   * it in device memory. */
   auto by_value = [&](auto blk) {
     memcpy(blk.pre, pre.data(), pre.size() * sizeof(uint64_t));
     spread(src, dst, m.step, P, total, P, -1, false, blk, s);
