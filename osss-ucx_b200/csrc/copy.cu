@@ -492,19 +492,20 @@ __global__ void __launch_bounds__(256, U > 2 ? 4 : 6)
 #pragma unroll 1
     for (int u = 0; u < U; u++) {
       const int t = tw + u * 512 + lane * 16;
-      /* at the row's ends part of a vector: its bytes [i0, i1) */
-      const int i0 = w.x0 + t < 0 ? a - t : 0;
-      const int i1 = t + 16 <= end ? 16 : (int)(end - t);
-      if (i1 <= i0) continue;
-      s = w.at(col, t + i0, &rem) - i0;
-      const uint4 x = meet16(s, s + w.jump, i0, rem < i1 - i0 ? i0 + rem : i1, i1);
-      if (i1 - i0 == 16) {
-        st16(row + t, x);
-      } else {
-        const unsigned wd[4] = {x.x, x.y, x.z, x.w};
-#pragma unroll
-        for (int i = 0; i < 16; i++)
-          if (i >= i0 && i < i1) row[t + i] = (char)(wd[i >> 2] >> (8 * (i & 3)));
+      if (w.x0 + t >= 0 && t + 16 <= end) {
+        s = w.at(col, t, &rem);
+        st16(row + t, meet16(s, s + w.jump, 0, rem < 16 ? rem : 16, 16));
+      } else if (t < end) {
+        /* the row's ends, byte by byte: put together like the others they cost
+         * the warps that cross blocks 5 to 17 %, and steps so small that their
+         * latency shows go by words */
+#pragma unroll 1
+        for (int i = 0; i < 16; i++) {
+          const int64_t y = w.x0 + t + i;
+          if (y < 0 || t + i >= end) continue;
+          const uint64_t k = (uint64_t)y / B;
+          row[t + i] = src0[j * B + k * step + ((uint64_t)y - k * B)];
+        }
       }
     }
   }
@@ -773,8 +774,8 @@ int alltoall_launch(int pe_start, int pe_stride, int P, uint64_t dest_off, uint6
   const uint64_t words = (uint64_t)P * P * nw;
   const bool flat = w == 16  ? nw >= 4 && words >= 70000 && !many
                     : w == 8 ? nw <= 128 || words <= 200000
-                    : w == 4 ? nw <= 12 || words <= 130000
-                             : words <= 100000;
+                    : w == 4 ? (nw <= 12 && words <= 1500000) || words <= 130000
+                             : words <= 120000;
   if (flat || B < 16) {
     const unsigned g = grid_for(words, 256, 8);
     switch (w) {

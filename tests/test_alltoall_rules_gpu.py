@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 GUARD = 64
 # common width -> block sizes around the lines (blocks of 4, 9 and 128 words;
-# steps of 70000, 100000, 130000 and 200000 words at these team sizes)
+# steps of 70000, 120000, 130000 and 200000 words at these team sizes)
 SIZES = {16: (16, 48, 64, 272, 496, 528, 2048), 8: (24, 456, 1016, 1032, 1400, 2056),
          4: (20, 36, 52, 116, 140, 1004), 2: (18, 30, 46, 94), 1: (17, 25, 45, 101)}
 
