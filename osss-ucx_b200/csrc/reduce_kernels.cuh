@@ -74,13 +74,15 @@ namespace {
  * over the elements the streaming kernel deferred (it left their dests
  * untouched, so in-place sources are still intact): one CTA per element
  * stages the P inputs in shared memory, then replays the algorithm's
- * operand order from there.  (Launched as a programmatic
- * dependent of the streaming kernel, its CTAs became resident on the few SMs
- * that kernel left free and stayed there: 256 members x 20000 floats with
- * NaNs throughout ran 16.1 ms, 5.8 as an ordinary launch; without any, 33.2
- * us either way.)  The last CTA to leave sets the counter back to zero for
- * the next call (every CTA reads it before it counts itself out), so no
- * memset precedes the streaming kernel. */
+ * operand order from there.  Launched as a programmatic dependent of the
+ * streaming kernel, whose CTAs let it start as they end (let_replay_start):
+ * its launch then costs a call without such elements next to nothing (2 to 3
+ * us otherwise), and its CTAs find the SMs empty.  (Let go as the streaming
+ * CTAs began, they piled up on the SMs that had room and stayed there: 256
+ * members x 20000 floats with NaNs throughout 16.1 ms, 6.2 so.)  The last CTA
+ * to leave sets the counter back to zero for the next call (every CTA reads
+ * it before it counts itself out), so no memset precedes the streaming
+ * kernel. */
 template <class T, int OP>
 __global__ void __launch_bounds__(256) k_minmax_fix(const RArgs a,
                                                     const unsigned long long *list,
@@ -89,6 +91,7 @@ __global__ void __launch_bounds__(256) k_minmax_fix(const RArgs a,
                                                     unsigned long long cap) {
   __shared__ T vals[fix_max_members<T>()];
   __shared__ T common;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const unsigned long long cnt = *(volatile unsigned long long *)count;
   const unsigned long long n = cnt < cap ? cnt : cap;
   for (unsigned long long k = blockIdx.x; k < n; k += gridDim.x) {
@@ -130,6 +133,12 @@ __global__ void __launch_bounds__(256) k_minmax_fix(const RArgs a,
       __threadfence();
     }
   }
+}
+
+/* This CTA no longer holds up the replay kernel that follows a MIN/MAX launch
+ * (which waits for this grid's results before it reads anything). */
+__device__ __forceinline__ void let_replay_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 /* ---- the streaming kernel ----------------------------------------------
@@ -559,6 +568,8 @@ k_reduce(const __grid_constant__ RArgs a) {
   }
   if constexpr (EDGES)
     reduce_edges<T, OP, ORDER, V, MM, C, POW2>(a, ln, lgG, nwarps - 1 - warp, nwarps);
+  if constexpr (MM)
+    if (a.fix_list != nullptr) let_replay_start();
 }
 
 /* CTAs of 256 threads of `kernel` that one SM holds at once (cached per
@@ -738,8 +749,18 @@ int run(const RArgs &base, cudaStream_t s) {
   }
   if constexpr (MM) {
     if (a.fix_list == nullptr) return B200SHM_OK;
-    k_minmax_fix<T, OP><<<2 * grid_sms(), 256, 0, s>>>(base, base.fix_list, base.fix_count,
-                                                      base.fix_done, base.fix_cap);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * grid_sms());
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    B200_CK(cudaLaunchKernelEx(&cfg, k_minmax_fix<T, OP>, base,
+                               (const unsigned long long *)base.fix_list, base.fix_count,
+                               base.fix_done, base.fix_cap));
     count_launch();
   }
   return B200SHM_OK;
