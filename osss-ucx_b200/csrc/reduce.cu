@@ -35,6 +35,8 @@ static int reduce_check(int op, int dtype, int algo, int pe_size) {
   if ((op <= B200SHM_XOR && !is_int) || ((op == B200SHM_MIN || op == B200SHM_MAX) && is_cpx))
     return fail(B200SHM_ERR_UNSUPPORTED, "reduce: op %d is not defined on dtype %d", op, dtype);
   if (pe_size < 1) return fail(B200SHM_ERR_ARG, "reduce: team size %d < 1", pe_size);
+  if (pe_size > kMaxMembers)
+    return fail(B200SHM_ERR_UNSUPPORTED, "reduce: more than %d members", kMaxMembers);
   int p2s = 1;
   while (p2s <= pe_size / 2) p2s *= 2;
   const bool tree = !is_int && op != B200SHM_MIN && op != B200SHM_MAX && algo != B200SHM_LINEAR;

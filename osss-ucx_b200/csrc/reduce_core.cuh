@@ -444,12 +444,17 @@ __device__ __forceinline__ bool p2s_extra(int q, int P, int p2s) {
   return (long long)(as + 1) * p2s / P == q;
 }
 
-/* The first of lane g's leaves where 2^lgG lanes share n: lane g has
- * [lane_leaf(g), lane_leaf(g + 1)).  64-bit products: integer and linear
- * reductions over buffers of the caller's have up to 2^31 - 1 members. */
-__host__ __device__ __forceinline__ int lane_leaf(int g, int n, int lgG) {
-  return (int)(((unsigned long long)g * (unsigned)n) >> lgG);
+/* Lanes (log2) that may share n members, at most `lg`: a lane's share begins
+ * at lane x n / lanes, in an int, which integer and linear reductions over
+ * buffers of the caller's, of up to kMaxMembers members, would overflow.
+ * (64-bit products in the kernel, or quotient and remainder apart, cost the
+ * byte-wide instances 10 to 15 %.) */
+constexpr int kMaxMembers = 0x7fffffff - 64; /* a round of loads past the last fits an int */
+inline int lanes_within_int(int lg, int n) {
+  while (lg > 0 && (long long)n << lg > 0x7fffffffll) lg--;
+  return lg;
 }
+__host__ __device__ __forceinline__ int lane_leaf(int g, int n, int lgG) { return (g * n) >> lgG; }
 
 constexpr int kMaxLevels = 13; /* trees of up to 4096 leaves */
 

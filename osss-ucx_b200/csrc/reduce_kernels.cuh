@@ -274,8 +274,8 @@ __device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, ui
       constexpr bool kOne = C == 0; /* one lane: bounds that the whole launch shares */
       const char *p = src + (kOne ? 0 : (uint64_t)l0 * a.sstep);
       r = ld_col<T, V, MODE>(p);
-      unsigned j = kOne ? 1 : (unsigned)l0 + 1; /* end may be the largest int: j + 8 is above */
-      const unsigned end = (unsigned)(kOne ? P : l1);
+      int j = kOne ? 1 : l0 + 1;
+      const int end = kOne ? P : l1; /* at most kMaxMembers: j + 8 fits an int */
       do { /* once at least: a MIN/MAX lane looks at its first operand below the loads */
         PK x[8];
         const uint64_t step = opaque(a.sstep);
@@ -284,7 +284,7 @@ __device__ __forceinline__ bool reduce_column(const RArgs &a, const Lane &ln, ui
           if (j + u < end) x[u] = ld_col<T, V, MODE>(p + (uint64_t)(u + 1) * step);
         p += 8 * step;
         if constexpr (MM)
-          if (j == (kOne ? 1 : (unsigned)l0 + 1)) cls = mm_flags<OP>(r);
+          if (j == (kOne ? 1 : l0 + 1)) cls = mm_flags<OP>(r);
 #pragma unroll
         for (int u = 0; u < 8; u++)
           if (j + u < end) {
@@ -688,7 +688,7 @@ int lanes_log2(uint64_t cols, int leaves, bool wide, int run) {
     while (lg < 4 && (4 << (lg + 1)) <= leaves &&
            (cols << (2 * lg)) < (uint64_t)grid_sms() * 128)
       lg++;
-  return lg;
+  return lanes_within_int(lg, leaves);
 }
 
 template <class T, int OP, int ORDER, bool MM, int MODE>

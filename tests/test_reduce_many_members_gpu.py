@@ -5,7 +5,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("members", [(1 << 27) - 1, 1 << 27, (1 << 28) + 3])
+@pytest.mark.parametrize("members", [(1 << 27) - 1, 1 << 27, (1 << 27) + 5])
 def test_one_byte_of_each_member_in_place(B, members):
     import torch
     pad = 256
