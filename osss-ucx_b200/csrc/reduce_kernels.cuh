@@ -491,11 +491,10 @@ __device__ __forceinline__ void reduce_edges(const RArgs &a, const Lane &ln, int
  *   code for single elements costs registers, so rows of whole packs, nedge
  *   == 0, have an instance without it), with extra members 3 (80), with a
  *   stack 2;
- *   complex PROD, four temporaries an element: 4 up to 16 leaves, 3 at 32
- *   (64 members x 409600 complex float: 76 us; 84 at 48 registers, which
- *   spills, 91 at 84, two CTAs), 2 beyond;
- *   chains in one lane as many as at the widths below, chains in several
- *   lanes 5 for 8-byte elements, 4 for their MIN/MAX (a compare and two
+ *   complex PROD, four temporaries an element, 4 (at 48 registers its trees
+ *   spill 160 to 250 bytes);
+ *   chains in one lane 4, for 1- and 2-byte elements what their unpacking
+ *   takes; chains in several lanes 5 for 8-byte elements, 4 for their MIN/MAX (a compare and two
  *   selects) and for 4-byte ones, 3 for MIN/MAX/PROD of 2-byte elements, 2
  *   for the others of 2 bytes and for bytes (which are unpacked into a
  *   register each: bytes' MIN/MAX and bit operations spill 180 to 420 bytes
@@ -514,14 +513,15 @@ constexpr int min_ctas() {
   if (ORDER == ORD_CHAIN && C == 0) {
     if (es == 1) return prod || OP == B200SHM_SUM ? 2 : 1;
     if (es == 2) return order || prod ? 3 : 2;
-    return es == 4 || std::is_same<T, cf32>::value || (cplx && prod) ? 3 : 4;
+    if (MODE == kElements && cplx) return 5;
+    return std::is_same<T, cf64>::value && prod ? 3 : 4;
   }
   if (ORDER == ORD_CHAIN) {
     if (es < 4) return es == 2 && (order || prod) ? 3 : 2;
     return es == 4 || EDGES || order ? 4 : 5;
   }
-  if (C == 0 || C < -3) return 2;
-  if (cplx && prod) return C > 32 ? 2 : !POW2 || C == 32 || C < 0 ? 3 : 4;
+  if (C == 0 || C < -3 || (C < 0 && MODE == kBytes)) return 2;
+  if (cplx && prod && POW2 && MODE != kElements) return 4;
   return !POW2 ? 3 : EDGES || C > 32 || MODE == kBytes ? 4 : 5;
 }
 template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2, int MODE, bool EDGES>
@@ -592,14 +592,15 @@ int resident_ctas(const void *kernel) {
 /* Launch over `lanes` threads of work.  Grid: up to 8 waves of the CTAs one
  * SM holds at once (B200SHM_REDUCE_WAVES overrides it, or
  * B200SHM_REDUCE_CTAS_PER_SM gives a fixed count); for chains in one lane 8
- * CTAs an SM (8 members x 2^21 int32: 19.6 us, 21.3 with 8 waves).  On the 64-PE x 2^20
+ * CTAs an SM where the sources are less than 128 MiB (8 members x 2^21 int32:
+ * 19.6 us, 21.3 with 8 waves; x 6.5 x 10^6 67.4 and 65.6).  On the 64-PE x 2^20
  * workload one exact wave was slowest (5.27 TB/s over the six reductions):
  * CTAs of a grid-stride loop finish unevenly and leave their SM's slots
  * idle, while the CTAs of later waves backfill them.  4 waves gave 5.73,
  * 6-16 waves 5.78-5.80, one pack per lane 5.76.  CTAs of 256 threads, less
  * where that leaves SMs without one. */
-template <bool ONE_LANE, class K>
-void launch_one(K kernel, uint64_t lanes, cudaStream_t s, const RArgs &a) {
+template <class K>
+void launch_one(K kernel, uint64_t lanes, bool small, cudaStream_t s, const RArgs &a) {
   static int per_sm_env = -1, waves = 8;
   if (per_sm_env < 0) {
     const char *e = getenv("B200SHM_REDUCE_CTAS_PER_SM");
@@ -611,8 +612,8 @@ void launch_one(K kernel, uint64_t lanes, cudaStream_t s, const RArgs &a) {
   int threads = 256;
   while (threads > 64 && lanes < sms * (uint64_t)threads) threads >>= 1;
   const int per_sm = per_sm_env ? per_sm_env
-                     : ONE_LANE ? 8
-                                : waves * resident_ctas((const void *)kernel);
+                     : small ? 8
+                             : waves * resident_ctas((const void *)kernel);
   kernel<<<grid_for(lanes, threads, per_sm), threads, 0, s>>>(a);
   count_launch();
 }
@@ -620,14 +621,15 @@ void launch_one(K kernel, uint64_t lanes, cudaStream_t s, const RArgs &a) {
 /* the instance with or without edges */
 template <class T, int OP, int ORDER, int V, bool MM, int C, bool POW2, int MODE>
 void launch_edges(uint64_t lanes, cudaStream_t s, const RArgs &a) {
-  constexpr bool one = ORDER == ORD_CHAIN && C == 0;
+  const bool small = ORDER == ORD_CHAIN && C == 0 &&
+                     a.N * sizeof(T) * (uint64_t)a.P < (128ull << 20);
   if constexpr (V > 1) {
     if (a.nedge) {
-      launch_one<one>(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, true>, lanes, s, a);
+      launch_one(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, true>, lanes, small, s, a);
       return;
     }
   }
-  launch_one<one>(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, false>, lanes, s, a);
+  launch_one(k_reduce<T, OP, ORDER, V, MM, C, POW2, MODE, false>, lanes, small, s, a);
 }
 
 /* Whether a lane has instances of 64 and 128 leaves (not long double, whose
@@ -675,8 +677,8 @@ void launch_tree(int n, uint64_t lanes, cudaStream_t s, const RArgs &a) {
  * B200SHM_REDUCE_COOP sets the starting point (0 or 1 = one lane per
  * column). */
 template <int ORDER>
-int lanes_log2(uint64_t cols, int leaves, bool wide, int run) {
-  int G = wide ? 1 : 2; /* 16-byte elements: a chain of one lane per element */
+int lanes_log2(uint64_t cols, int leaves, bool one, int run) {
+  int G = one ? 1 : 2; /* 16-byte elements, say: a chain of one lane per element */
   if (ORDER != ORD_CHAIN) G = std::max(2, std::min(8, leaves / run));
   static const char *ec = getenv("B200SHM_REDUCE_COOP"); /* read once */
   if (ec) G = std::max(1, std::min(8, atoi(ec)));
@@ -703,8 +705,12 @@ void run_mode(RArgs &a, cudaStream_t s) {
   constexpr bool any_order = ORDER == ORD_CHAIN && (std::is_integral<T>::value || MM);
   const bool split = any_order || ORDER == ORD_BUTTERFLY || (ORDER == ORD_BINOMIAL && pow2);
   const bool long_runs = kLongRuns<T, MODE> && (leaves >= 256 || (pow2 && a.nedge == 0));
-  const int run = long_runs ? 128 : 32;
-  a.lgG = split ? lanes_log2<ORDER>(a.nvec + a.nedge, leaves, sizeof(T) == 16, run) : 0;
+  /* single elements of 4 bytes: longer runs, and of 1 byte: one lane, else a
+   * warp reads less than a sector of each member (250 members x 209715 floats
+   * 218 -> 119 us, 130 x 1613193 bytes 316 -> 233) */
+  const int run = long_runs ? 128 : MODE == kElements && sizeof(T) == 4 ? 64 : 32;
+  const bool one = sizeof(T) == 16 || (MODE == kElements && sizeof(T) == 1);
+  a.lgG = split ? lanes_log2<ORDER>(a.nvec + a.nedge, leaves, one, run) : 0;
   const uint64_t lanes = std::max<uint64_t>(a.nvec + a.nedge, 1) << a.lgG;
   if constexpr (ORDER == ORD_CHAIN && any_order) {
     if (MM || a.lgG) launch_edges<T, OP, ORDER, V, MM, 1, true, MODE>(lanes, s, a);
@@ -735,7 +741,7 @@ int run(const RArgs &base, cudaStream_t s) {
   /* few narrow elements off the grid: what counts is lanes, and an element a
    * lane makes V times as many (bytes, MAX over 8 members x 8193: 2.1 us, 3.8
    * in packs; over 2 x 32769 2.0 and 2.6; 8 x 524289 the other way round) */
-  const bool few = sizeof(T) <= 2 && (dp & 15) && a.N <= 65536;
+  const bool few = sizeof(T) <= 2 && (dp & 15) && a.N * (uint64_t)a.P <= 262144;
   if (((sp ^ dp) & 15) == 0 && (steps & 15) == 0 && dp % sizeof(T) == 0 && !few) {
     /* the packs begin at a 128-byte line of the dest, so that warps do not
      * share lines (vectors shorter than a few lines: at the 16-byte grid) */
