@@ -553,15 +553,9 @@ __device__ __forceinline__ Pack<T, V> shfl_pack(const Pack<T, V> &v, int lane) {
   return shfl_words(v, [lane](uint32_t x) { return __shfl_sync(0xffffffffu, x, lane); });
 }
 template <class T, int V>
-__device__ __forceinline__ Pack<T, V> shfl_xor_any(const Pack<T, V> &v, int m) {
+__device__ __forceinline__ Pack<T, V> shfl_xor_pack(const Pack<T, V> &v, int m) {
   return shfl_words(v, [m](uint32_t x) { return __shfl_xor_sync(0xffffffffu, x, m); });
 }
-
-template <class T, int V>
-__device__ __forceinline__ Pack<T, V> shfl_xor_pack(const Pack<T, V> &v, int m) {
-  return shfl_xor_any(v, m);
-}
-
 
 /* The exact replay inside a warp, for teams whose butterfly has at most
  * kExactLeaves leaves: V elements from e0 at a time, every lane holding the
@@ -631,7 +625,7 @@ __device__ __noinline__ void exact_columns(const RArgs &a, uint64_t e0) {
 #pragma unroll
       for (int k = 0; k < K; k++) {
         if (m < 32) {
-          o[k] = shfl_xor_any(v[k], m);
+          o[k] = shfl_xor_pack(v[k], m);
         } else {
           o[k] = v[k];
 #pragma unroll
