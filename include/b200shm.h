@@ -316,9 +316,11 @@ int b200shm_span_amo(int amo, int dtype, int G, const uint64_t *bases, int pe_st
 
 /* One reduction of a batch: the arguments of b200shm_reduce.  `lanes` and
  * `tile` are outputs of b200shm_batch_create: the lanes per 16-byte column
- * and the units per tile, at most, the autotuner chose (0 = this reduction runs as
- * its own launch because the batch kernels do not cover its
- * (dtype, op, algo, size)); `algo` is rewritten when it was AUTO. */
+ * and the tile size the autotuner chose (0 = this reduction runs as its own
+ * launch because the batch kernels do not cover its (dtype, op, algo,
+ * size)).  A tile has that many units, fewer for teams of more than 8 (so
+ * that tiles read about the same bytes), but always one pass of a CTA over
+ * its columns.  `algo` is rewritten when it was AUTO. */
 typedef struct b200shm_reduce_desc {
   int32_t op, dtype, algo;
   int32_t pe_start, pe_stride, pe_size;
@@ -439,7 +441,8 @@ int b200shm_serve_enqueue(b200shm_server *srv, const b200shm_request *req,
 /* 1 when the request completed, 0 while it is pending, < 0 on an error.
  * *fetched (may be NULL) receives an AMO's old value, and for the other
  * kinds the dest offset the request wrote to (the one the loop allocated,
- * for B200SHM_SERVE_ALLOC). */
+ * for B200SHM_SERVE_ALLOC).  It is there until the request queue_slots
+ * tickets later completes. */
 int b200shm_serve_poll(b200shm_server *srv, uint64_t ticket, uint64_t *fetched);
 /* Device clock stamps (globaltimer, ns) of a completed request still in
  * its slot: copied from the ring into device memory, its last tiles

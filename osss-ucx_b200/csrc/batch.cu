@@ -446,8 +446,8 @@ __device__ __forceinline__ void run_one(const BTile &d, const BPlan &p, uint32_t
   case kid_of(DS, OP_, ORD_BUTTERFLY, 1): run_one<F_, OP_, ORD_BUTTERFLY, false, 2>(t, p, nullptr); break;
 
 /* The order-free reductions, the left folds of the linear order, and the
- * butterflies of small teams (at most two leaves per lane): no stack, 64
- * registers, 4 CTAs per SM.  What bounds them is loads in flight, so the
+ * butterflies of small teams (at most two leaves per lane): no stack, held
+ * to 64 registers (24 bytes spill), 4 CTAs per SM.  What bounds them is loads in flight, so the
  * registers are kept down: a pointer per lane stepped from member to
  * member, one register for a column's operand classes.  One CTA per tile
  * (each starts with a 48-byte record of all it needs): CTAs start and end

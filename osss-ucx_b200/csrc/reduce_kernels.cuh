@@ -494,12 +494,12 @@ __device__ __forceinline__ void reduce_edges(const RArgs &a, const Lane &ln, int
  *   complex PROD, four temporaries an element, 4 (at 48 registers its trees
  *   spill 160 to 250 bytes);
  *   chains in one lane 4, for 1- and 2-byte elements what their unpacking
- *   takes; chains in several lanes 5 for 8-byte elements, 4 for their MIN/MAX (a compare and two
- *   selects) and for 4-byte ones, 3 for MIN/MAX/PROD of 2-byte elements, 2
- *   for the others of 2 bytes and for bytes (which are unpacked into a
- *   register each: bytes' MIN/MAX and bit operations spill 180 to 420 bytes
- *   there, and still ran 1.1 to 3 times as fast as the one CTA of 160 to 200
- *   registers that does not, over 24 to 256 members);
+ *   takes; chains in several lanes 5 for 8-byte elements, 4 for their MIN/MAX
+ *   (a compare and two selects) and for 4-byte ones, 3 for MIN/MAX/PROD of
+ *   2-byte elements, 2 for the others of 2 bytes and for bytes (which are
+ *   unpacked into a register each: bytes' MIN/MAX and bit operations spill
+ *   180 to 420 bytes there, and still ran 1.1 to 3 times as fast as the one
+ *   CTA of 160 to 200 registers that does not, over 24 to 256 members);
  *   3 for the float MIN/MAX ones: holding those to 64 registers (4 CTAs, no
  *   spills) measured slower on the 64-PE headline (f64 MAX 5908-5912 against
  *   5938-5950 GB/s). */
@@ -593,8 +593,8 @@ int resident_ctas(const void *kernel) {
  * SM holds at once (B200SHM_REDUCE_WAVES overrides it, or
  * B200SHM_REDUCE_CTAS_PER_SM gives a fixed count); for chains in one lane 8
  * CTAs an SM where the sources are less than 128 MiB (8 members x 2^21 int32:
- * 19.6 us, 21.3 with 8 waves; x 6.5 x 10^6 67.4 and 65.6).  On the 64-PE x 2^20
- * workload one exact wave was slowest (5.27 TB/s over the six reductions):
+ * 19.6 us, 21.3 with 8 waves; x 6.5 x 10^6 67.4 and 65.6).  On the 64-PE x
+ * 2^20 workload one exact wave was slowest (5.27 TB/s over the six reductions):
  * CTAs of a grid-stride loop finish unevenly and leave their SM's slots
  * idle, while the CTAs of later waves backfill them.  4 waves gave 5.73,
  * 6-16 waves 5.78-5.80, one pack per lane 5.76.  CTAs of 256 threads, less

@@ -268,7 +268,7 @@ constexpr unsigned kMirrorBatch = 256;
  * moves them past the requests at its start that have none left.
  * Block 0 looks for published requests before each claim, so that they are
  * copied while the others serve the batch before (2048 all-to-alls of 4
- * members x 64 KiB: 1727 -> 1595 us); with a heap budget it waits for the
+ * members x 64 KiB: 1727 -> 1590 us); with a heap budget it waits for the
  * batch to be handed out, as the others do. */
 __device__ int claim(const SArgs &a, SReq *req, unsigned long long *cr, unsigned long long *ct,
                      unsigned *count, unsigned long long *mfrom, unsigned long long *mupto,
@@ -1298,14 +1298,14 @@ int b200shm_serve_replay(b200shm_server *s, const b200shm_request *reqs, uint64_
     }
     return B200SHM_OK;
   }
-  /* Requests that have arrived are published up to kRun at a time; between
-   * such runs one pass looks over the outstanding completion words, each on
-   * a line of its own that the device wrote, so they are fetched ahead.  (One
-   * request at a time, three clock reads and two divisions for each: 2048
-   * fetch-adds 423 us, 353 now.)  A slot may be reused as
-   * soon as its request is complete, so a request waits until the completion
-   * that its slot holds has been read: else the loop, when it is as fast as
-   * this thread, overwrites it. */
+  /* Requests that have arrived are published up to kRun at a time, run after
+   * run while the ring has room; then one pass looks over the outstanding
+   * completion words, each on a line of its own that the device wrote, so
+   * they are fetched ahead.  (One request at a time, three clock reads and
+   * two divisions for each: 2048 fetch-adds 423 us, 353 now.)  A slot may be
+   * reused as soon as its request is complete, so a request waits until the
+   * completion that its slot holds has been read: else the loop, when it is
+   * as fast as this thread, overwrites it. */
   constexpr unsigned kRun = 16;
   struct Out {
     const SDone *d;
